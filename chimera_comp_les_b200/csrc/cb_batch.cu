@@ -387,6 +387,8 @@ int cb_batch_create(const cb_config *cfg, int nblocks, const int *dims, cb_batch
     set_sutherland(d, cfg->visT, cfg->tref, cfg->ren, cfg->gamma, cfg->ma);
     d.twod = cfg->twod;  // -twoD 1: no i-face fluxes
     d.gm1 = cfg->gamma - 1.0;
+    d.r_pr = 1. / cfg->pr;
+    d.r_gm1 = 1. / d.gm1;
     d.kheat = cfg->gamma / cfg->pr / (cfg->gamma - 1.0);
     d.nvq = 1;  // nvert starts zero
     d.calc_sigma = (cfg->les && cfg->calc_sigma) ? 1 : 0;

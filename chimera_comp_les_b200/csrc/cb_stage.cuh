@@ -27,7 +27,10 @@
 // once per node.  Each face flux is computed exactly once per plane.
 // Metrics, nvert and nu_t are read through the read-only cache.
 #pragma once
+#include <type_traits>
+
 #include "cb_common.cuh"
+#include "cb_div.cuh"
 
 namespace cb {
 
@@ -230,18 +233,18 @@ __device__ __forceinline__ R weno3_l(R qm, R q0, R qp) {
   const R d0 = R(0.6666667), d1 = R(0.3333333), eps = R(1e-6);  // rhs.c:2386 (truncated weights)
   R r0 = R(0.5) * q0 + R(0.5) * qp, r1 = R(-0.5) * qm + R(1.5) * q0;
   R b0 = (qp - q0) * (qp - q0), b1 = (qm - q0) * (qm - q0);
-  R a0 = d0 / ((eps + b0) * (eps + b0)), a1 = d1 / ((eps + b1) * (eps + b1));
-  R as = a0 + a1;
-  return (a0 / as) * r0 + (a1 / as) * r1;
+  const R a0 = Den<R>((eps + b0) * (eps + b0))(d0), a1 = Den<R>((eps + b1) * (eps + b1))(d1);
+  const Den<R> as(a0 + a1);
+  return as(a0) * r0 + as(a1) * r1;
 }
 template <typename R>
 __device__ __forceinline__ R weno3_r(R qm, R q0, R qp) {
   const R d0 = R(0.6666667), d1 = R(0.3333333), eps = R(1e-6);
   R r0 = R(1.5) * q0 - R(0.5) * qp, r1 = R(0.5) * qm + R(0.5) * q0;
   R b0 = (qp - q0) * (qp - q0), b1 = (qm - q0) * (qm - q0);
-  R a0 = d0 / ((eps + b0) * (eps + b0)), a1 = d1 / ((eps + b1) * (eps + b1));
-  R as = a0 + a1;
-  return (a0 / as) * r0 + (a1 / as) * r1;
+  const R a0 = Den<R>((eps + b0) * (eps + b0))(d0), a1 = Den<R>((eps + b1) * (eps + b1))(d1);
+  const Den<R> as(a0 + a1);
+  return as(a0) * r0 + as(a1) * r1;
 }
 template <typename R>
 __device__ __forceinline__ R eno_r(R qm, R q0, R qp, int k) {
@@ -273,10 +276,10 @@ __device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
   const R b0 = c13 * (t0 * t0) + R(0.25) * (u0 * u0);
   const R b1 = c13 * (t1 * t1) + R(0.25) * (u1 * u1);
   const R b2 = c13 * (t2 * t2) + R(0.25) * (u2 * u2);
-  const R a0 = R(0.1) / ((eps + b0) * (eps + b0));
-  const R a1 = R(0.6) / ((eps + b1) * (eps + b1));
-  const R a2 = R(0.3) / ((eps + b2) * (eps + b2));
-  return ((a0 * q0 + a1 * q1) + a2 * q2) / (R(6.0) * ((a0 + a1) + a2));
+  const R a0 = Den<R>((eps + b0) * (eps + b0))(R(0.1));
+  const R a1 = Den<R>((eps + b1) * (eps + b1))(R(0.6));
+  const R a2 = Den<R>((eps + b2) * (eps + b2))(R(0.3));
+  return Den<R>(R(6.0) * ((a0 + a1) + a2))((a0 * q0 + a1 * q1) + a2 * q2);
 }
 
 // Conserved state and pressure of one node as the ring stores them, from its
@@ -288,13 +291,17 @@ template <typename R, bool MIX>
 __device__ __forceinline__ void node_qp(const DevCfg &c, const double v[5], bool pst, double pin, R q[5], R &p) {
   double pp = 0.0, e = v[4];
   if (v[0] != 0.0) {
+    const Den<double> rho(v[0]);
     if (MIX) {
-      const double ri = 1.0 / v[0];
+      const double ri = rho(1.0);
       pp = (c.gamma - 1) * (v[4] - 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) * ri);
       e -= c.e_ref;
       pp -= c.p_ref;
     } else {
-      pp = pst ? pin : (c.gamma - 1) * (v[4] - 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) / v[0]);
+      const double ke = 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
+      double kr = rho(ke);
+      if (!finite_hi(kr)) kr = ke / v[0];
+      pp = pst ? pin : (c.gamma - 1) * (v[4] - kr);
     }
   }
 #pragma unroll
@@ -309,27 +316,45 @@ __device__ __forceinline__ void node_qp(const DevCfg &c, const double v[5], bool
 // face velocity measure 0.5*(uconL + uconR) that multiplies H_ref.
 // The mixed form multiplies by one reciprocal of each state's density
 // instead of dividing by it four times (FP32 rounding differences only).
+// One side's face velocity and sound speed sqrt(|gamma p / rho| h.h) by a / b
+// and sqrt: where the branch-free quotients and roots leave their range (zero
+// or non-finite density or sound speed).
+static __device__ __noinline__ double2 side_speed_ieee(double r, double ru, double rv, double rw, double p, double h0,
+                                                       double h1, double h2) {
+  const double u = h0 * (ru / r) + h1 * (rv / r) + h2 * (rw / r);
+  const double cc = GAMMA_CONV * p / r, gii = h0 * h0 + h1 * h1 + h2 * h2;
+  return make_double2(u, sqrt(fabs(cc) * gii));
+}
 template <typename R, bool MIX>
 __device__ __forceinline__ void rusanov(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
                                         bool r_from_l, R pref, R F[5], R &Uf) {
-  R uconL, uconR, cL, cR;
+  R uconL, uconR, saL, saR;
+  const R gii = h[0] * h[0] + h[1] * h[1] + h[2] * h[2];
   if constexpr (MIX) {
     const R ril = R(1) / QL[0], rir = R(1) / QR[0];
     const R UR = (h[0] * QR[1] + h[1] * QR[2] + h[2] * QR[3]) * rir;
     uconL = use_qr_for_l ? UR : (h[0] * QL[1] + h[1] * QL[2] + h[2] * QL[3]) * ril;
     uconR = r_from_l ? uconL : UR;
-    cL = R(GAMMA_CONV) * (pL + pref) * ril;
-    cR = R(GAMMA_CONV) * (pR + pref) * rir;
+    const R cL = R(GAMMA_CONV) * (pL + pref) * ril;
+    const R cR = R(GAMMA_CONV) * (pR + pref) * rir;
+    saL = fabs(uconL) + sqrt(fabs(cL) * gii);
+    saR = fabs(uconR) + sqrt(fabs(cR) * gii);
   } else {
-    uconL = use_qr_for_l ? (h[0] * (QR[1] / QR[0]) + h[1] * (QR[2] / QR[0]) + h[2] * (QR[3] / QR[0]))
-                         : (h[0] * (QL[1] / QL[0]) + h[1] * (QL[2] / QL[0]) + h[2] * (QL[3] / QL[0]));
-    uconR = r_from_l ? uconL : (h[0] * (QR[1] / QR[0]) + h[1] * (QR[2] / QR[0]) + h[2] * (QR[3] / QR[0]));
-    cL = R(GAMMA_CONV) * pL / QL[0];
-    cR = R(GAMMA_CONV) * pR / QR[0];
+    const Den<R> rl(QL[0]), rr(QR[0]);
+    const R UR = h[0] * rr(QR[1]) + h[1] * rr(QR[2]) + h[2] * rr(QR[3]);
+    uconL = use_qr_for_l ? UR : h[0] * rl(QL[1]) + h[1] * rl(QL[2]) + h[2] * rl(QL[3]);
+    uconR = r_from_l ? uconL : UR;
+    saL = fabs(uconL) + root(fabs(rl(R(GAMMA_CONV) * pL)) * gii);
+    saR = fabs(uconR) + root(fabs(rr(R(GAMMA_CONV) * pR)) * gii);
+    if (!(finite_hi(saL) && finite_hi(saR))) {
+      const double2 l = side_speed_ieee(QL[0], QL[1], QL[2], QL[3], pL, h[0], h[1], h[2]);
+      const double2 r = side_speed_ieee(QR[0], QR[1], QR[2], QR[3], pR, h[0], h[1], h[2]);
+      uconL = use_qr_for_l ? r.x : l.x;
+      uconR = r_from_l ? uconL : r.x;
+      saL = fabs(uconL) + l.y;
+      saR = fabs(uconR) + r.y;
+    }
   }
-  R gii = h[0] * h[0] + h[1] * h[1] + h[2] * h[2];
-  R saL = fabs(uconL) + sqrt(fabs(cL) * gii);
-  R saR = fabs(uconR) + sqrt(fabs(cR) * gii);
   R SA = (saL < saR) ? saR : saL;
   F[0] = R(0.5) * (QL[0] * uconL + QR[0] * uconR) - R(0.5) * SA * (QR[0] - QL[0]);
 #pragma unroll
@@ -346,25 +371,40 @@ __device__ __forceinline__ void rusanov(const R QL[5], const R QR[5], R pL, R pR
 // Roe-averaged Jacobian along n = h/|h|, acoustic speeds below 0.1 c~
 // smoothed to (l^2 + delta^2) / (2 delta).  Mixed form: the enthalpy adds
 // back H_ref; pressure and energy differences are shift-free.
-template <typename R, bool MIX>
-__device__ __forceinline__ void roe(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
-                                    bool r_from_l, R pref, R href, R F[5], R &Uf) {
-  (void)pref;
+// The FP64 form's quotients and roots are the branch-free ones (cb_div.cuh);
+// IEEE: a / b and sqrt, for the states where those leave their range.
+template <typename R>
+struct PlainDen {
+  R b;
+  __device__ __forceinline__ explicit PlainDen(R b_) : b(b_) {}
+  __device__ __forceinline__ R operator()(R a) const { return a / b; }
+};
+template <typename R, bool MIX, bool IEEE>
+__device__ __forceinline__ void roe_flux(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
+                                         bool r_from_l, R href, R F[5], R &Uf) {
   const R g = R(GAMMA_CONV);
+  using D = std::conditional_t<IEEE || MIX, PlainDen<R>, Den<R>>;
+  auto rt_of = [](R x) -> R {
+    if constexpr (IEEE || MIX) return sqrt(x);
+    else return root(x);
+  };
+  const D dl(QL[0]), dr_(QR[0]);
   // the mixed form multiplies by reciprocals of the densities, the face area
   // and the root sum (FP32 rounding differences only)
   const R ril = MIX ? R(1) / QL[0] : R(0), rir = MIX ? R(1) / QR[0] : R(0);
-#define CB_DIVL(x) (MIX ? (x) * ril : (x) / QL[0])
-#define CB_DIVR(x) (MIX ? (x) * rir : (x) / QR[0])
+#define CB_DIVL(x) (MIX ? (x) * ril : dl(x))
+#define CB_DIVR(x) (MIX ? (x) * rir : dr_(x))
   R uconL = use_qr_for_l ? (h[0] * CB_DIVR(QR[1]) + h[1] * CB_DIVR(QR[2]) + h[2] * CB_DIVR(QR[3]))
                          : (h[0] * CB_DIVL(QL[1]) + h[1] * CB_DIVL(QL[2]) + h[2] * CB_DIVL(QL[3]));
   R uconR = r_from_l ? uconL : (h[0] * CB_DIVR(QR[1]) + h[1] * CB_DIVR(QR[2]) + h[2] * CB_DIVR(QR[3]));
-  const R area = sqrt(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
+  const R area = rt_of(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
   const R ria = MIX ? R(1) / area : R(0);
-  const R nx = MIX ? h[0] * ria : h[0] / area, ny = MIX ? h[1] * ria : h[1] / area, nz = MIX ? h[2] * ria : h[2] / area;
-  const R sl = sqrt(QL[0]), sr = sqrt(QR[0]);
+  const D da(area);
+  const R nx = MIX ? h[0] * ria : da(h[0]), ny = MIX ? h[1] * ria : da(h[1]), nz = MIX ? h[2] * ria : da(h[2]);
+  const R sl = rt_of(QL[0]), sr = rt_of(QR[0]);
   const R ris = MIX ? R(1) / (sl + sr) : R(0);
-  const R wl = MIX ? sl * ris : sl / (sl + sr), wr = MIX ? sr * ris : sr / (sl + sr);
+  const D ds(sl + sr);
+  const R wl = MIX ? sl * ris : ds(sl), wr = MIX ? sr * ris : ds(sr);
   const R uL = CB_DIVL(QL[1]), vL = CB_DIVL(QL[2]), zL = CB_DIVL(QL[3]);
   const R uR = CB_DIVR(QR[1]), vR = CB_DIVR(QR[2]), zR = CB_DIVR(QR[3]);
   const R HL = CB_DIVL(MIX ? (QL[4] + pL + href) : (QL[4] + pL));
@@ -373,28 +413,61 @@ __device__ __forceinline__ void roe(const R QL[5], const R QR[5], R pL, R pR, co
 #undef CB_DIVR
   const R rt = sl * sr, ut = wl * uL + wr * uR, vt = wl * vL + wr * vR, zt = wl * zL + wr * zR;
   const R Ht = wl * HL + wr * HR, q2 = ut * ut + vt * vt + zt * zt;
-  const R c2 = (g - R(1.0)) * (Ht - R(0.5) * q2), ct = sqrt(fabs(c2));
+  const R c2 = (g - R(1.0)) * (Ht - R(0.5) * q2), ct = rt_of(fabs(c2));
   const R Unt = ut * nx + vt * ny + zt * nz;
   const R dp = pR - pL, dr = QR[0] - QL[0];
   const R du = uR - uL, dv = vR - vL, dz = zR - zL, dUn = du * nx + dv * ny + dz * nz;
-  const R a1 = (dp - rt * ct * dUn) / (R(2.0) * c2), a2 = dr - dp / c2, a3 = (dp + rt * ct * dUn) / (R(2.0) * c2);
+  const D dc2(c2), d2c2(R(2.0) * c2);
+  const R a1 = d2c2(dp - rt * ct * dUn), a2 = dr - dc2(dp), a3 = d2c2(dp + rt * ct * dUn);
   R l1 = fabs(Unt - ct), l2 = fabs(Unt), l3 = fabs(Unt + ct);
   const R delta = R(0.1) * ct;
   if (l1 < delta) l1 = (l1 * l1 + delta * delta) / (R(2.0) * delta);
   if (l3 < delta) l3 = (l3 * l3 + delta * delta) / (R(2.0) * delta);
   const R s1 = l1 * a1, s2 = l2 * a2, s3 = l3 * a3, ss = l2 * rt;
-  R D[5];
-  D[0] = s1 + s2 + s3;
-  D[1] = s1 * (ut - ct * nx) + s2 * ut + s3 * (ut + ct * nx) + ss * (du - dUn * nx);
-  D[2] = s1 * (vt - ct * ny) + s2 * vt + s3 * (vt + ct * ny) + ss * (dv - dUn * ny);
-  D[3] = s1 * (zt - ct * nz) + s2 * zt + s3 * (zt + ct * nz) + ss * (dz - dUn * nz);
-  D[4] = s1 * (Ht - Unt * ct) + s2 * R(0.5) * q2 + s3 * (Ht + Unt * ct) + ss * (ut * du + vt * dv + zt * dz - Unt * dUn);
-  F[0] = R(0.5) * (QL[0] * uconL + QR[0] * uconR) - R(0.5) * area * D[0];
+  R D5[5];
+  D5[0] = s1 + s2 + s3;
+  D5[1] = s1 * (ut - ct * nx) + s2 * ut + s3 * (ut + ct * nx) + ss * (du - dUn * nx);
+  D5[2] = s1 * (vt - ct * ny) + s2 * vt + s3 * (vt + ct * ny) + ss * (dv - dUn * ny);
+  D5[3] = s1 * (zt - ct * nz) + s2 * zt + s3 * (zt + ct * nz) + ss * (dz - dUn * nz);
+  D5[4] = s1 * (Ht - Unt * ct) + s2 * R(0.5) * q2 + s3 * (Ht + Unt * ct) + ss * (ut * du + vt * dv + zt * dz - Unt * dUn);
+  F[0] = R(0.5) * (QL[0] * uconL + QR[0] * uconR) - R(0.5) * area * D5[0];
 #pragma unroll
   for (int a = 0; a < 3; a++)
-    F[1 + a] = R(0.5) * ((QL[1 + a] * uconL + QR[1 + a] * uconR) + (pL * h[a] + pR * h[a])) - R(0.5) * area * D[1 + a];
-  F[4] = R(0.5) * ((pL + QL[4]) * uconL + (pR + QR[4]) * uconR) - R(0.5) * area * D[4];
+    F[1 + a] = R(0.5) * ((QL[1 + a] * uconL + QR[1 + a] * uconR) + (pL * h[a] + pR * h[a])) - R(0.5) * area * D5[1 + a];
+  F[4] = R(0.5) * ((pL + QL[4]) * uconL + (pR + QR[4]) * uconR) - R(0.5) * area * D5[4];
   Uf = MIX ? R(0.5) * (uconL + uconR) : R(0);
+}
+struct RoeIn {
+  double QL[5], QR[5], pL, pR, h[3];
+  bool use_qr_for_l, r_from_l;
+};
+struct RoeOut {
+  double F[5];
+};
+static __device__ __noinline__ RoeOut roe_ieee(const RoeIn in) {
+  RoeOut o;
+  double uf;
+  roe_flux<double, false, true>(in.QL, in.QR, in.pL, in.pR, in.h, in.use_qr_for_l, in.r_from_l, 0.0, o.F, uf);
+  return o;
+}
+template <typename R, bool MIX>
+__device__ __forceinline__ void roe(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
+                                    bool r_from_l, R href, R F[5], R &Uf) {
+  roe_flux<R, MIX, false>(QL, QR, pL, pR, h, use_qr_for_l, r_from_l, href, F, Uf);
+  if constexpr (!MIX) {
+    if (!(finite_hi(F[0]) && finite_hi(F[1]) && finite_hi(F[2]) && finite_hi(F[3]) && finite_hi(F[4]))) {
+      RoeIn in;
+#pragma unroll
+      for (int q = 0; q < 5; q++) { in.QL[q] = QL[q]; in.QR[q] = QR[q]; }
+#pragma unroll
+      for (int q = 0; q < 3; q++) in.h[q] = h[q];
+      in.pL = pL; in.pR = pR;
+      in.use_qr_for_l = use_qr_for_l; in.r_from_l = r_from_l;
+      const RoeOut o = roe_ieee(in);
+#pragma unroll
+      for (int q = 0; q < 5; q++) F[q] = o.F[q];
+    }
+  }
 }
 
 // ------------------------------------------------------- inviscid face ----
@@ -573,12 +646,12 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
       }
     }
     if (LES) {
-      if (ROE) roe<R, MIX>(QL, QR, pL, pR, h, false, false, pref, href, Fw, Ufw);
+      if (ROE) roe<R, MIX>(QL, QR, pL, pR, h, false, false, href, Fw, Ufw);
       else rusanov<R, MIX>(QL, QR, pL, pR, h, false, false, pref, Fw, Ufw);
     } else {
       const bool use_qr_l = !PLAIN && (pos == m - 2 && bc_hi(c, d) == 1);
       const bool r_from_l = !PLAIN && (pos == 0 && bc_lo(c, d) == 1);
-      if (ROE) roe<R, MIX>(QL, QR, pL, pR, h, use_qr_l, r_from_l, pref, href, Fw, Ufw);
+      if (ROE) roe<R, MIX>(QL, QR, pL, pR, h, use_qr_l, r_from_l, href, Fw, Ufw);
       else rusanov<R, MIX>(QL, QR, pL, pR, h, use_qr_l, r_from_l, pref, Fw, Ufw);
     }
   }
@@ -607,12 +680,13 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
 #pragma unroll
     for (int s = 0; s < 4; s++) {
       const MetV<R> ms = s == 1 ? m0 : (s == 2 ? m1 : met_load<R, MIX>(F, d, g0 + (s - 1) * sd));
-      U[s] = R(1.) / Q[s][0] * (ms.x * Q[s][1] + ms.y * Q[s][2] + ms.z * Q[s][3]);
+      U[s] = Den<R>(Q[s][0])(R(1.)) * (ms.x * Q[s][1] + ms.y * Q[s][2] + ms.z * Q[s][3]);
       EP[s] = P[s] + Q[s][4];
     }
+    const Den<R> third = den_const<R>(R(3.0), R(1.0 / 3.0));
     const R fp4 = R(1.0) / R(12.0) * (-P[0] + R(7) * P[1] + R(7) * P[2] - P[3]);
     if (c.central == 2) {
-#define CB_FP2(A0, A1, A2, A3) ((A1 + A2) * (U[1] + U[2]) / R(3.0) - R(1.) / R(24.) * (A0 * U[0] + A0 * U[2] + A1 * U[1] + A1 * U[3] + A2 * U[2] + A2 * U[0] + A3 * U[1] + A3 * U[3]))
+#define CB_FP2(A0, A1, A2, A3) (third((A1 + A2) * (U[1] + U[2])) - R(1.) / R(24.) * (A0 * U[0] + A0 * U[2] + A1 * U[1] + A1 * U[3] + A2 * U[2] + A2 * U[0] + A3 * U[1] + A3 * U[3]))
       Fcen[0] = CB_FP2(Q[0][0], Q[1][0], Q[2][0], Q[3][0]);
       Fcen[1] = CB_FP2(Q[0][1], Q[1][1], Q[2][1], Q[3][1]) + fp4 * h[0];
       Fcen[2] = CB_FP2(Q[0][2], Q[1][2], Q[2][2], Q[3][2]) + fp4 * h[1];
@@ -633,7 +707,7 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
   } else {
     const R rc = R(0.5) * (Q[1][0] + Q[2][0]), uc = R(0.5) * (Q[1][1] + Q[2][1]), vc = R(0.5) * (Q[1][2] + Q[2][2]);
     const R wc = R(0.5) * (Q[1][3] + Q[2][3]), ec = R(0.5) * (Q[1][4] + Q[2][4]);
-    const R Uc = (h[0] * uc + h[1] * vc + h[2] * wc) / rc;
+    const R Uc = Den<R>(rc)(h[0] * uc + h[1] * vc + h[2] * wc);
     const R pa = R(0.5) * (P[1] + P[2]);
     Fcen[0] = rc * Uc;
     Fcen[1] = uc * Uc + pa * h[0];
@@ -800,9 +874,15 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
     for (int q = 0; q < 3; q++) uh[q] = R(0.5) * (Rg.get(F_U + q, b) + Rg.get(F_U + q, a));
   }
   if (!PLAIN && c.twod == 1) uh[0] = R(0.);
-  const R gm = R(c.gamma);
+  R heat;
+  if constexpr (MIX) {
+    heat = nu * R(c.kheat);
+  } else {  // gamma * nu / Pr / (gamma - 1)
+    heat = Den<double>(c.gm1, c.r_gm1)(Den<double>(c.pr, c.r_pr)(c.gamma * nu));
+    if (!finite_hi(heat)) heat = c.gamma * nu / c.pr / c.gm1;
+  }
   Fv[4] = (Fv[1] * uh[0] + Fv[2] * uh[1] + Fv[3] * uh[2]) +
-          (g11 * dpdc + g21 * dpde + g31 * dpdz) * ajc * (MIX ? nu * R(c.kheat) : gm * nu / R(c.pr) / R(c.gm1));
+          (g11 * dpdc + g21 * dpde + g31 * dpdz) * ajc * heat;
 
   A[0] = A[1] = A[2] = R(0.);
   if (LES) {  // rhs.c:1677-1710
@@ -831,7 +911,7 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
       const R tx = (tu - div * md0) * ajc * (nut * rho_c);
       const R ty = (tv - div * md1) * ajc * (nut * rho_c);
       const R tz = (tw - div * md2) * ajc * (nut * rho_c);
-      const R sgs = -S2 * pf * R(c.ci) * R(2.0) / R(3.0);
+      const R sgs = den_const<R>(R(3.0), R(1.0 / 3.0))(-S2 * pf * R(c.ci) * R(2.0));
       A[0] = tx + sgs * md0 * rho_c * sigma_c;
       A[1] = ty + sgs * md1 * rho_c * sigma_c;
       A[2] = tz + sgs * md2 * rho_c * sigma_c;
@@ -1115,19 +1195,28 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
           // one FP64 reciprocal instead of five divisions: the products differ
           // from the quotients by at most an FP64 ulp, far below the FP32
           // rounding of the shifted values stored next
-          const double ri = 1.0 / r;
+          const double ri = Den<double>(r)(1.0);
           v[F_P] = (c.gamma - 1) * (v[4] - 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) * ri);
           v[F_U] = v[1] * ri;
           v[F_V] = v[2] * ri;
           v[F_W] = v[3] * ri;
           v[F_T] = v[F_P] * ri;
         } else {  // the reference's quotients (EqOfState rhs.c:4850, CalcUCat rhs.c:1349)
-          v[F_P] = pst ? stg[pslot * PN + idx]
-                       : (c.gamma - 1) * (v[4] - 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) / r);
-          v[F_U] = v[1] / r;
-          v[F_V] = v[2] / r;
-          v[F_W] = v[3] / r;
-          v[F_T] = v[F_P] / r;
+          const Den<double> rho(r);
+          const double ke = 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
+          const double pc = pst ? stg[pslot * PN + idx] : 0.;
+          v[F_P] = pst ? pc : (c.gamma - 1) * (v[4] - rho(ke));
+          v[F_U] = rho(v[1]);
+          v[F_V] = rho(v[2]);
+          v[F_W] = rho(v[3]);
+          v[F_T] = rho(v[F_P]);
+          if (!(finite_hi(v[F_U]) && finite_hi(v[F_V]) && finite_hi(v[F_W]) && finite_hi(v[F_T]))) {
+            v[F_P] = pst ? pc : (c.gamma - 1) * (v[4] - ke / r);
+            v[F_U] = v[1] / r;
+            v[F_V] = v[2] / r;
+            v[F_W] = v[3] / r;
+            v[F_T] = v[F_P] / r;
+          }
         }
         if (MIX) {
           v[F_RE] -= c.e_ref;
