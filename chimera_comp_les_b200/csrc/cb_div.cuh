@@ -17,10 +17,10 @@
 // chains of a face's quotients overlap.  The square root is the same
 // correction of a Goldschmidt iterate (none of 1.05e9 differed from
 // __dsqrt_rn).  Measured per time step, before and after, with bit-identical
-results: MUSCL + Rusanov 128^3 1.50 -> 1.36 ms, WENO3 blend 97x75x61
-1.60 -> 1.00 ms, WENO5-JS + Roe 96^3 4.22 -> 2.86 ms, inviscid WENO5-JS +
-Rusanov 64^3 1.08 -> 0.63 ms; mixed form (the node reciprocal only) WENO5-JS
-+ Roe 192^3 7.97 -> 7.85 ms.
+// results: MUSCL + Rusanov 128^3 1.50 -> 1.36 ms, WENO3 blend 97x75x61
+// 1.60 -> 1.00 ms, WENO5-JS + Roe 96^3 4.22 -> 2.86 ms, inviscid WENO5-JS +
+// Rusanov 64^3 1.08 -> 0.63 ms; mixed form (the node reciprocal only) WENO5-JS
+// + Roe 192^3 7.97 -> 7.85 ms.
 //
 // Range: a zero, infinite, subnormal or NaN denominator (or a zero or
 // infinite radicand) gives NaN; callers for which that state can lead to a
