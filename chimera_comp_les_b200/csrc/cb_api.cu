@@ -622,15 +622,17 @@ int cb_create(const cb_config *cfg, cb_ctx **out) {
   cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream);
   if (fill_ptab(c)) return bail(CB_E_CUDA, "pointer table");
   // k-chunk: whole waves of the resident blocks (1 per SM in the FP64 form,
-  // 2 in the mixed form); a chunk's prologue costs about one plane.  The
-  // autotuner (cb_autotune) refines this by measurement.
+  // 2 in the mixed form); a chunk's prologue costs about one plane.  Small
+  // blocks take chunks down to one plane: 32^3 FP64 44.2 us per stage at
+  // k-chunk 4, 30.2 at 2; mixed 30.7 at 4, 21.0 at 1.  The autotuner
+  // (cb_autotune) refines this by measurement.
   {
     const int by = cfg->weno_order == 5 ? SBY_W5 : BY;
     const int tiles = ((cfg->mx - 2 + BX - 1) / BX) * ((cfg->my - 2 + by - 1) / by);
     const int nk = cfg->mz - 2;
     const int slots = c->sms * (cfg->precision == CB_MIXED ? 2 : 1);
     double best = 1e30;
-    for (int kc = 4; kc <= nk; kc++) {
+    for (int kc = 1; kc <= nk; kc++) {
       const int chunks = (nk + kc - 1) / kc;
       const long long blocks = (long long)tiles * chunks;
       const long long waves = (blocks + slots - 1) / slots;

@@ -85,10 +85,11 @@ struct StageGeo {
 };
 
 // Threads of a stage-kernel block.  The FP64 form runs two threads per face:
-// the first NT compute the faces' inviscid fluxes, the next NT their viscous
-// and SGS fluxes, so each thread holds half the live FP64 values and a block
-// of 2 NT threads fits the register file (16 warps per SM at 32 x 7 instead of
-// 8).  The mixed form keeps one thread per face and two blocks per SM.
+// inviscid fluxes and viscous and SGS fluxes are formed in different threads
+// (plane_faces deals them to the block's two halves), so each thread holds
+// half the live FP64 values and a block of 2 NT threads fits the register file
+// (16 warps per SM at 32 x 7 instead of 8).  The mixed form keeps one thread
+// per face and two blocks per SM.
 template <int FLUX, bool MIX>
 struct StageThreads {
   static constexpr bool SPLIT = !MIX;
@@ -947,25 +948,19 @@ __device__ __forceinline__ void face_flux(const DevCfg &c, const DevFields &F, c
   G[AOFF] = A[0]; G[AOFF + 1] = A[1]; G[AOFF + 2] = A[2];
 }
 
-// The inviscid half (G[0..4]) or the viscous and SGS half (G[VOFF..VOFF+4],
-// G[AOFF..AOFF+2]) of face_flux, for the FP64 form's two threads per face;
-// the same calls, so the same values.
+// The inviscid part (G[0..4]) or the viscous and SGS part (G[VOFF..VOFF+4],
+// G[AOFF..AOFF+2]) of face_flux: the FP64 form's jobs; the same calls, so the
+// same values.
 template <typename R, bool MIX, bool LES, bool VISC, class RG, int DIR, int FLUX = 0, bool NV0 = false>
 __device__ __forceinline__ void face_flux_half(const DevCfg &c, const DevFields &F, const RG &Rg, NRef a, int fi,
-                                               int fj, int k, int drt, int role, R *G) {
+                                               int fj, int k, int drt, bool conv, R *G) {
   constexpr int VOFF = FaceWidth<MIX>::VOFF, AOFF = FaceWidth<MIX>::AOFF;
   static_assert(!MIX, "the mixed form stores visc - conv per face");
-  if (role == 0) {
+  if (conv) {
     conv_face<R, MIX, LES, RG, DIR, FLUX, NV0>(c, F, Rg, a, fi, fj, k, drt, G);
-  } else {
+  } else if constexpr (VISC) {
     R Fv[5], A[3];
-    if (VISC) {
-      visc_face<R, MIX, LES, RG, DIR, NV0, FLUX>(c, F, Rg, a, fi, fj, k, drt, Fv, A);
-    } else {
-#pragma unroll
-      for (int q = 0; q < 5; q++) Fv[q] = R(0.);
-      A[0] = A[1] = A[2] = R(0.);
-    }
+    visc_face<R, MIX, LES, RG, DIR, NV0, FLUX>(c, F, Rg, a, fi, fj, k, drt, Fv, A);
 #pragma unroll
     for (int q = 0; q < 5; q++) G[VOFF + q] = Fv[q];
     G[AOFF] = A[0]; G[AOFF + 1] = A[1]; G[AOFF + 2] = A[2];
@@ -1016,104 +1011,135 @@ static_assert(2 * (STAGE_SMEM_BYTES_MIXED + 1024) <= 233472, "mixed form: two bl
 static_assert(2 * (StageSmem<float, true, false, true>::bytes + 1024) <= 233472, "WENO5 mixed: two blocks per SM");
 static_assert(2 * (StageSmem<float, true, true, false>::bytes + 1024) <= 233472, "mixed with the metric slot: two blocks per SM");
 
+// Face u of direction d of a tile: its node A (tile reference a, global fi,
+// fj) and whether the direction has it.
+template <class G>
+__device__ __forceinline__ bool face_node(int d, int u, int i0, int j0, int &fi, int &fj, NRef &a) {
+  constexpr int BX = G::BX;
+  if (d == 0) {
+    const int fx = u % (BX + 1), fy = u / (BX + 1);
+    fi = i0 - 1 + fx; fj = j0 + fy;
+    a = NRef{0, fy + 2, fx + 1};
+    return u < G::NXF;
+  }
+  const int fx = u % BX, fy = u / BX;
+  fi = i0 + fx;
+  if (d == 1) {
+    fj = j0 - 1 + fy;
+    a = NRef{0, fy + 1, fx + 2};
+    return u < G::NYF;
+  }
+  fj = j0 + fy;
+  a = NRef{0, fy + 2, fx + 2};
+  return u < G::NZF;
+}
+
 // All face fluxes of plane k of a tile into the face buffers (ZONLY: just the
 // k-faces, for the prologue).  A function rather than a lambda so that it is
 // always inlined: an outlined call would copy the kernel parameters to local
 // memory.
 // With the metric slot (StageMet) the k-face comes back in gzr (registers:
 // thread u of the k round is the thread that updates node u); otherwise it
-// goes to gzb (the FP64 form forms the two halves of a face in two threads).
+// goes to gzb.
+//
+// FP64 form: the plane is six jobs, the inviscid (c0-c2) and the viscous and
+// SGS (v0-v2) fluxes of the three directions, each for the NT threads of one
+// half of the block.  Both halves wait at the end of the plane, so the jobs
+// are dealt by weight.  Measured against the inviscid jobs in one half and the
+// viscous ones in the other (per step):
+//   default         c0 c1 v0 | c2 v1 v2        inviscid jobs somewhat heavier;
+//                   MUSCL 128^3 1.31 -> 1.25 ms, WENO3 blend 97x75x61 0.97 -> 0.92,
+//                   sigma 1 with the dynamic model 96x80x72 0.94 -> 0.92
+//   WENO5-JS        c0 c1 | c2 v0 v1 v2        an inviscid job about 3.5 viscous
+//                   ones (barrier stall 4.0 of 11.4 cycles per issue before);
+//                   96^3 + Roe 2.86 -> 2.06 ms
+//   no viscous flux c0, rows of c2 | c1, the other rows of c2
+//                   WENO5-JS 64^3 0.63 -> 0.50 ms
+constexpr unsigned JOBS_C0 = 1, JOBS_C1 = 2, JOBS_C2 = 3, JOBS_V0 = 4, JOBS_V1 = 5, JOBS_V2 = 6;
+template <bool VISC, int FLUX>
+__device__ __forceinline__ unsigned plane_jobs(int role, bool zonly) {
+  if (zonly) return role == 0 ? JOBS_C2 : (VISC ? JOBS_V2 : 0u);
+  if (!VISC) return role == 0 ? JOBS_C0 | JOBS_C2 << 4 : JOBS_C1 | JOBS_C2 << 4;
+  if ((FLUX & FLUX_W5) != 0) return role == 0 ? JOBS_C0 | JOBS_C1 << 4 : JOBS_C2 | JOBS_V0 << 4 | JOBS_V1 << 8 | JOBS_V2 << 12;
+  return role == 0 ? JOBS_C0 | JOBS_C1 << 4 | JOBS_V0 << 8 : JOBS_C2 | JOBS_V1 << 4 | JOBS_V2 << 8;
+}
+
 template <typename R, bool MIX, bool LES, bool VISC, bool ZONLY, int FLUX, bool NV0, class RG>
 __device__ __forceinline__ void plane_faces(const DevCfg &c, const DevFields &F, const RG &Rg, int i0, int j0, int k,
                                             R *gxb, R *gyb, R *gzb, R *gzr) {
   using G = StageGeo<FLUX>;
-  constexpr int BX = G::BX, NT = G::NT, NG = FaceWidth<MIX>::NG;
-  constexpr bool SPLIT = StageThreads<FLUX, MIX>::SPLIT;
+  constexpr int NT = G::NT, NG = FaceWidth<MIX>::NG;
   constexpr int VOFF = FaceWidth<MIX>::VOFF;
   const int tid = threadIdx.x;
-  // role 0: the faces' inviscid fluxes; role 1 (FP64 form): their viscous
-  // and SGS fluxes (warp-uniform: NT is a multiple of 32)
-  const int role = SPLIT ? tid / NT : 0;
+  if constexpr (StageThreads<FLUX, MIX>::SPLIT) {
+    const int role = tid / NT;  // the half of the block (warp-uniform: NT is a multiple of 32)
 #pragma unroll 1
-  for (int r = ZONLY ? 2 : 0; r < 3; r++) {
-    const int u = SPLIT ? tid - role * NT : tid;  // face index within this round's direction
-    int d, fi, fj;
-    NRef a;
-    R *dst;
-    int nslot;
-    if (r == 0) {
-      d = 0;
-      if (u >= G::NXF) continue;
-      const int fx = u % (BX + 1), fy = u / (BX + 1);
-      fi = i0 - 1 + fx; fj = j0 + fy;
-      a = NRef{0, fy + 2, fx + 1};
-      dst = gxb; nslot = G::NXF;
-    } else if (r == 1) {
-      d = 1;
-      if (u >= G::NYF) continue;
-      const int fx = u % BX, fy = u / BX;
-      fi = i0 + fx; fj = j0 - 1 + fy;
-      a = NRef{0, fy + 1, fx + 2};
-      dst = gyb; nslot = G::NYF;
-    } else {
-      d = 2;
-      if (u >= G::NZF) continue;
-      const int fx = u % BX, fy = u / BX;
-      fi = i0 + fx; fj = j0 + fy;
-      a = NRef{0, fy + 2, fx + 2};
-      dst = gzb; nslot = G::NZF;
-    }
-    R Gf[NG];
-    // -twoD 1 forms no i-face flux (rhs.c:1487, 2646, 3465): it stays zero
-    const bool live = fi <= c.mx - 2 && fj <= c.my - 2 && !(d == 0 && (FLUX & FLUX_PLAIN) == 0 && c.twod == 1);
-    if constexpr (SPLIT) {
-      // this thread's half of the face: G[0..4], or G[VOFF..NG-1]
-      const int q0 = role == 0 ? 0 : VOFF, q1 = role == 0 ? VOFF : NG;
-      if (live) {
+    for (unsigned list = plane_jobs<VISC, FLUX>(role, ZONLY); list; list >>= 4) {
+      const int job = (int)(list & 15u) - 1;
+      const bool conv = job < 3;
+      const int d = conv ? job : job - 3;
+      int u = tid - role * NT;
+      if (!VISC && !ZONLY && d == 2) {  // the k-faces' rows shared by the two halves
+        constexpr int CUT = (G::NZF / 32 + 1) / 2 * 32;
+        if (role == 0 && u >= CUT) continue;
+        if (role == 1) u += CUT;
+      }
+      int fi, fj;
+      NRef a;
+      if (!face_node<G>(d, u, i0, j0, fi, fj, a)) continue;
+      R *dst = d == 0 ? gxb : (d == 1 ? gyb : gzb);
+      const int nslot = d == 0 ? G::NXF : (d == 1 ? G::NYF : G::NZF);
+      R Gf[NG];
+#pragma unroll
+      for (int q = 0; q < NG; q++) Gf[q] = R(0.);
+      // -twoD 1 forms no i-face flux (rhs.c:1487, 2646, 3465): it stays zero
+      if (fi <= c.mx - 2 && fj <= c.my - 2 && !(d == 0 && (FLUX & FLUX_PLAIN) == 0 && c.twod == 1)) {
         // one instantiation per direction (d is warp-uniform): the index
         // arithmetic of every stencil shift folds into constants (4 % faster
         // than one copy for all directions at 128 registers); the WENO5-JS
         // variants, at 168 registers, keep one copy (13 % faster there)
         if constexpr ((FLUX & FLUX_W5) != 0)
-          face_flux_half<R, MIX, LES, VISC, RG, -1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, role, Gf);
-        else if (d == 0) face_flux_half<R, MIX, LES, VISC, RG, 0, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, role, Gf);
-        else if (d == 1) face_flux_half<R, MIX, LES, VISC, RG, 1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, role, Gf);
-        else face_flux_half<R, MIX, LES, VISC, RG, 2, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, role, Gf);
+          face_flux_half<R, MIX, LES, VISC, RG, -1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, conv, Gf);
+        else if (d == 0) face_flux_half<R, MIX, LES, VISC, RG, 0, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, conv, Gf);
+        else if (d == 1) face_flux_half<R, MIX, LES, VISC, RG, 1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, conv, Gf);
+        else face_flux_half<R, MIX, LES, VISC, RG, 2, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, conv, Gf);
+      }
+      if (conv) {
+#pragma unroll
+        for (int q = 0; q < VOFF; q++) dst[(size_t)q * nslot + u] = Gf[q];
       } else {
 #pragma unroll
-        for (int q = 0; q < NG; q++) Gf[q] = R(0.);
+        for (int q = VOFF; q < NG; q++) dst[(size_t)q * nslot + u] = Gf[q];
       }
-#pragma unroll
-      for (int q = 0; q < NG; q++)
-        if (q >= q0 && q < q1) dst[(size_t)q * nslot + u] = Gf[q];
-      continue;
     }
-    if (live) {
-      if constexpr (MIX) {
+  } else {
+#pragma unroll 1
+    for (int d = ZONLY ? 2 : 0; d < 3; d++) {
+      int fi, fj;
+      NRef a;
+      if (!face_node<G>(d, tid, i0, j0, fi, fj, a)) continue;
+      R *dst = d == 0 ? gxb : (d == 1 ? gyb : gzb);
+      const int nslot = d == 0 ? G::NXF : (d == 1 ? G::NYF : G::NZF);
+      R Gf[NG];
+      if (fi <= c.mx - 2 && fj <= c.my - 2 && !(d == 0 && (FLUX & FLUX_PLAIN) == 0 && c.twod == 1)) {
         // one instantiation per direction (d is warp-uniform): 16 % faster
         // for the FP32 arithmetic of the mixed form
         if (d == 0) face_flux<R, MIX, LES, VISC, RG, 0, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, Gf);
         else if (d == 1) face_flux<R, MIX, LES, VISC, RG, 1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, Gf);
         else face_flux<R, MIX, LES, VISC, RG, 2, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, Gf);
       } else {
-        // one copy for all directions: the FP64 form at 255 registers runs
-        // 12 % slower with three
-        face_flux<R, MIX, LES, VISC, RG, -1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, Gf);
+#pragma unroll
+        for (int q = 0; q < NG; q++) Gf[q] = R(0.);
       }
-    } else {
+      if (StageMet<MIX, NV0, FLUX>::on && d == 2) {
 #pragma unroll
-      for (int q = 0; q < NG; q++) Gf[q] = R(0.);
+        for (int q = 0; q < NG; q++) gzr[q] = Gf[q];
+        continue;
+      }
+#pragma unroll
+      for (int q = 0; q < NG; q++) dst[(size_t)q * nslot + tid] = Gf[q];
     }
-    if (StageMet<MIX, NV0, FLUX>::on && r == 2) {
-#pragma unroll
-      for (int q = 0; q < NG; q++) gzr[q] = Gf[q];
-      continue;
-    }
-#pragma unroll
-    for (int q = 0; q < NG; q++) dst[(size_t)q * nslot + u] = Gf[q];
   }
-  (void)NT;
-  (void)VOFF;
   (void)gzb;
 }
 
@@ -1184,11 +1210,11 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
   };
   // staging -> ring slot s with the derived p, u, v, w, T (EqOfState rhs.c:4850,
   // CalcUCat rhs.c:1349), all in FP64; the mixed form stores shifted FP32 values
-  auto derive = [&](int s) {
-    for (int idx = SPLIT ? tid - HT : tid; idx < PN && idx >= 0; idx += HT) {
+  auto derive_node = [&](int s, int idx, const double *raw, int rstride, double nvn, double pn) {
+    {
       double v[NF];
 #pragma unroll
-      for (int q = 0; q < 5; q++) v[q] = stg[q * PN + idx];
+      for (int q = 0; q < 5; q++) v[q] = raw[q * rstride];
       if (v[0] != 0.0) {
         const double r = v[0];
         if (MIX) {
@@ -1204,14 +1230,13 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
         } else {  // the reference's quotients (EqOfState rhs.c:4850, CalcUCat rhs.c:1349)
           const Den<double> rho(r);
           const double ke = 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
-          const double pc = pst ? stg[pslot * PN + idx] : 0.;
-          v[F_P] = pst ? pc : (c.gamma - 1) * (v[4] - rho(ke));
+          v[F_P] = pst ? pn : (c.gamma - 1) * (v[4] - rho(ke));
           v[F_U] = rho(v[1]);
           v[F_V] = rho(v[2]);
           v[F_W] = rho(v[3]);
           v[F_T] = rho(v[F_P]);
           if (!(finite_hi(v[F_U]) && finite_hi(v[F_V]) && finite_hi(v[F_W]) && finite_hi(v[F_T]))) {
-            v[F_P] = pst ? pc : (c.gamma - 1) * (v[4] - ke / r);
+            v[F_P] = pst ? pn : (c.gamma - 1) * (v[4] - ke / r);
             v[F_U] = v[1] / r;
             v[F_V] = v[2] / r;
             v[F_W] = v[3] / r;
@@ -1236,8 +1261,12 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
 #pragma unroll
         for (int q = 0; q < NF; q++) base[(size_t)q * PN] = R(v[q]);
       }
-      if (nvs) nvc[s * PN + idx] = (unsigned char)(stg[5 * PN + idx] * 4.0);
+      if (nvs) nvc[s * PN + idx] = (unsigned char)(nvn * 4.0);
     }
+  };
+  auto derive = [&](int s) {
+    for (int idx = SPLIT ? tid - HT : tid; idx < PN && idx >= 0; idx += HT)
+      derive_node(s, idx, stg + idx, PN, nvs ? stg[5 * PN + idx] : 0., pst ? stg[pslot * PN + idx] : 0.);
   };
   // async copy of plane kk's FP32 metric vectors and nu_t over the slot's
   // node box into the slot (SMET)
@@ -1255,29 +1284,57 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
       cp_async_commit();
     }
   };
-  auto load_plane_sync = [&](int kk, int s) {
-    issue_stage(kk);
-    cp_async_wait_all();
-    __syncthreads();
-    derive(s);
-    __syncthreads();
-  };
-
   // prologue: planes kb-1-H .. kb+H in slots 0 .. NPL-1, k-face kb-1/2 (its
-  // stencil is exactly those planes), then plane kb+H+1 into slot 0
+  // stencil is exactly those planes), then plane kb+H+1 into slot 0.  All
+  // planes' copies are in flight at once, the raw state straight into the ring
+  // (a node's five doubles take the place of its own fields) and its nvert and
+  // carried pressure into the idle face buffers; the thread that copied a node
+  // derives it, so one wait covers the prologue's loads (one plane after the
+  // other, their latencies added up to about half a plane of the march: with
+  // this 128^3 MUSCL mixed 0.274 -> 0.270 ms, FP64 0.644 -> 0.612 ms per stage
+  // at k-chunk 7, 32^3 FP64 30.2 -> 27.0 us at k-chunk 2).
+  constexpr int NTB = StageThreads<FLUX, MIX>::N;
+  double *aux = reinterpret_cast<double *>(gxb);  // [NPL][2][PN]: nvert, lP
+  static_assert(sizeof(R) * NG * (size_t)(NXF + NYF + (SMET ? 0 : NZF)) >=
+                    sizeof(double) * (size_t)PN * ((size_t)NPL * (NV0 ? 0 : 1) + (MIX ? 0 : NPL)),
+                "the face buffers hold the prologue's nvert and lP planes");
+  constexpr int AUXP = NV0 ? 0 : NPL * PN;  // first lP plane
+  constexpr int RS = RG::AOS ? 1 : PN;      // stride of a node's raw doubles in the ring
+  auto raw_node = [&](int e) {
+    const int t = e / PN, idx = e - t * PN;
+    return RG::AOS ? reinterpret_cast<double *>(Rg.pl) + (size_t)e * 5
+                   : reinterpret_cast<double *>(Rg.pl) + (size_t)t * NF * PN + idx;
+  };
   Rg.sb = 0;
   issue_met(kb - 1);  // the metric slot holds plane kb-1 for the prologue's k-face
-#pragma unroll 1
-  for (int t = 0; t < NPL; t++) load_plane_sync(kb - 1 - H + t, t);
+  for (int e = tid; e < NPL * PN; e += NTB) {
+    const int t = e / PN, idx = e - t * PN, ly = idx / PX, lx = idx - ly * PX;
+    const int kk = kb - 1 - H + t, xi = i0 - 2 + lx, yj = j0 - 2 + ly;
+    const bool ok = kk >= -2 && kk <= c.mz + 1 && xi <= c.mx + 1 && yj <= c.my + 1;
+    const long long go = ok ? gidx(c, xi, yj, kk) : 0;  // src-size 0 below: nothing is read
+    double *raw = raw_node(e);
+#pragma unroll
+    for (int q = 0; q < 5; q++) cp_async8(raw + q * RS, F.q[q] + go, ok);
+    if (nvs) cp_async8(aux + e, F.nvert + go, ok);
+    if (pst) cp_async8(aux + AUXP + e, F.pin + go, ok);
+  }
+  issue_stage(kb + H + 1);
+  cp_async_wait_all();
+  for (int e = tid; e < NPL * PN; e += NTB) {
+    const int t = e / PN;
+    derive_node(t, e - t * PN, raw_node(e), RS, nvs ? aux[e] : 0., pst ? aux[AUXP + e] : 0.);
+  }
+  __syncthreads();
   R gzr[NG];  // with the metric slot: k-face k+1/2 of the node this thread updates
   plane_faces<R, MIX, LES, VISC, true, FLUX, NV0>(c, F, Rg, i0, j0, kb - 1, gxb, gyb, gzb, gzr);  // k-face kb-1/2
   __syncthreads();
   R Gzp[NG];  // k-face k-1/2 of the node this thread updates
 #pragma unroll
   for (int q = 0; q < NG; q++) Gzp[q] = uact ? (SMET ? gzr[q] : gzb[(size_t)q * NZF + tid]) : R(0.);
-  __syncthreads();
   issue_met(kb);
-  load_plane_sync(kb + H + 1, 0);
+  derive(0);
+  if (SMET) cp_async_wait_all();
+  __syncthreads();
   int base = 1;  // slot of plane k-H
 
   for (int k = kb; k < ke; k++) {
