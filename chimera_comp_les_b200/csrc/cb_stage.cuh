@@ -332,14 +332,14 @@ __device__ __forceinline__ void rusanov(const R QL[5], const R QR[5], R pL, R pR
   R uconL, uconR, saL, saR;
   const R gii = h[0] * h[0] + h[1] * h[1] + h[2] * h[2];
   if constexpr (MIX) {
-    const R ril = R(1) / QL[0], rir = R(1) / QR[0];
+    const R ril = rcp_approx(QL[0]), rir = rcp_approx(QR[0]);
     const R UR = (h[0] * QR[1] + h[1] * QR[2] + h[2] * QR[3]) * rir;
     uconL = use_qr_for_l ? UR : (h[0] * QL[1] + h[1] * QL[2] + h[2] * QL[3]) * ril;
     uconR = r_from_l ? uconL : UR;
     const R cL = R(GAMMA_CONV) * (pL + pref) * ril;
     const R cR = R(GAMMA_CONV) * (pR + pref) * rir;
-    saL = fabs(uconL) + sqrt(fabs(cL) * gii);
-    saR = fabs(uconR) + sqrt(fabs(cR) * gii);
+    saL = fabs(uconL) + root(fabs(cL) * gii);
+    saR = fabs(uconR) + root(fabs(cR) * gii);
   } else {
     const Den<R> rl(QL[0]), rr(QR[0]);
     const R UR = h[0] * rr(QR[1]) + h[1] * rr(QR[2]) + h[2] * rr(QR[3]);
@@ -378,33 +378,35 @@ template <typename R>
 struct PlainDen {
   R b;
   __device__ __forceinline__ explicit PlainDen(R b_) : b(b_) {}
+  __device__ __forceinline__ PlainDen doubled() const { return PlainDen(R(2.0) * b); }
   __device__ __forceinline__ R operator()(R a) const { return a / b; }
 };
 template <typename R, bool MIX, bool IEEE>
 __device__ __forceinline__ void roe_flux(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
                                          bool r_from_l, R href, R F[5], R &Uf) {
   const R g = R(GAMMA_CONV);
-  using D = std::conditional_t<IEEE || MIX, PlainDen<R>, Den<R>>;
+  using D = std::conditional_t<IEEE, PlainDen<R>, Den<R>>;
   auto rt_of = [](R x) -> R {
-    if constexpr (IEEE || MIX) return sqrt(x);
+    if constexpr (IEEE) return sqrt(x);
     else return root(x);
   };
   const D dl(QL[0]), dr_(QR[0]);
   // the mixed form multiplies by reciprocals of the densities, the face area
   // and the root sum (FP32 rounding differences only)
-  const R ril = MIX ? R(1) / QL[0] : R(0), rir = MIX ? R(1) / QR[0] : R(0);
+  const R ril = MIX ? dl(R(1)) : R(0), rir = MIX ? dr_(R(1)) : R(0);
 #define CB_DIVL(x) (MIX ? (x) * ril : dl(x))
 #define CB_DIVR(x) (MIX ? (x) * rir : dr_(x))
   R uconL = use_qr_for_l ? (h[0] * CB_DIVR(QR[1]) + h[1] * CB_DIVR(QR[2]) + h[2] * CB_DIVR(QR[3]))
                          : (h[0] * CB_DIVL(QL[1]) + h[1] * CB_DIVL(QL[2]) + h[2] * CB_DIVL(QL[3]));
   R uconR = r_from_l ? uconL : (h[0] * CB_DIVR(QR[1]) + h[1] * CB_DIVR(QR[2]) + h[2] * CB_DIVR(QR[3]));
-  const R area = rt_of(h[0] * h[0] + h[1] * h[1] + h[2] * h[2]);
-  const R ria = MIX ? R(1) / area : R(0);
+  const R hh = h[0] * h[0] + h[1] * h[1] + h[2] * h[2], area = rt_of(hh);
   const D da(area);
+  R ria = R(0);
+  if constexpr (MIX) ria = rsqrt_approx(hh);
   const R nx = MIX ? h[0] * ria : da(h[0]), ny = MIX ? h[1] * ria : da(h[1]), nz = MIX ? h[2] * ria : da(h[2]);
   const R sl = rt_of(QL[0]), sr = rt_of(QR[0]);
-  const R ris = MIX ? R(1) / (sl + sr) : R(0);
   const D ds(sl + sr);
+  const R ris = MIX ? ds(R(1)) : R(0);
   const R wl = MIX ? sl * ris : ds(sl), wr = MIX ? sr * ris : ds(sr);
   const R uL = CB_DIVL(QL[1]), vL = CB_DIVL(QL[2]), zL = CB_DIVL(QL[3]);
   const R uR = CB_DIVR(QR[1]), vR = CB_DIVR(QR[2]), zR = CB_DIVR(QR[3]);
@@ -418,7 +420,7 @@ __device__ __forceinline__ void roe_flux(const R QL[5], const R QR[5], R pL, R p
   const R Unt = ut * nx + vt * ny + zt * nz;
   const R dp = pR - pL, dr = QR[0] - QL[0];
   const R du = uR - uL, dv = vR - vL, dz = zR - zL, dUn = du * nx + dv * ny + dz * nz;
-  const D dc2(c2), d2c2(R(2.0) * c2);
+  const D dc2(c2), d2c2 = dc2.doubled();
   const R a1 = d2c2(dp - rt * ct * dUn), a2 = dr - dc2(dp), a3 = d2c2(dp + rt * ct * dUn);
   R l1 = fabs(Unt - ct), l2 = fabs(Unt), l3 = fabs(Unt + ct);
   const R delta = R(0.1) * ct;
@@ -684,7 +686,6 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
       U[s] = Den<R>(Q[s][0])(R(1.)) * (ms.x * Q[s][1] + ms.y * Q[s][2] + ms.z * Q[s][3]);
       EP[s] = P[s] + Q[s][4];
     }
-    const Den<R> third = den_const<R>(R(3.0), R(1.0 / 3.0));
     const R fp4 = R(1.0) / R(12.0) * (-P[0] + R(7) * P[1] + R(7) * P[2] - P[3]);
     if (c.central == 2) {
 #define CB_FP2(A0, A1, A2, A3) (third((A1 + A2) * (U[1] + U[2])) - R(1.) / R(24.) * (A0 * U[0] + A0 * U[2] + A1 * U[1] + A1 * U[3] + A2 * U[2] + A2 * U[0] + A3 * U[1] + A3 * U[3]))
@@ -912,7 +913,7 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
       const R tx = (tu - div * md0) * ajc * (nut * rho_c);
       const R ty = (tv - div * md1) * ajc * (nut * rho_c);
       const R tz = (tw - div * md2) * ajc * (nut * rho_c);
-      const R sgs = den_const<R>(R(3.0), R(1.0 / 3.0))(-S2 * pf * R(c.ci) * R(2.0));
+      const R sgs = third(-S2 * pf * R(c.ci) * R(2.0));
       A[0] = tx + sgs * md0 * rho_c * sigma_c;
       A[1] = ty + sgs * md1 * rho_c * sigma_c;
       A[2] = tz + sgs * md2 * rho_c * sigma_c;
