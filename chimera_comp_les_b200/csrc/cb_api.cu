@@ -160,12 +160,10 @@ static int flux_bits(const cb_ctx *c) {
     if (f.s_x == 1.0) fl |= FLUX_SIGMA1;
     else if (f.s_x == 0.0) fl |= FLUX_SIGMA0;
   }
-  // every face periodic or an interface, no 2-D mode, MUSCL (or WENO5-JS,
-  // whose reconstruction the W5 bit selects): the PLAIN variants
-  bool per = f.twod == 0 && (f.fluxorder == 2 || f.weno_order == 5);
+  // every face periodic: the PLAIN variants
+  bool per = true;
   for (int s = 0; s < 6; s++) per = per && f.bctype[s] == 7;
-  if (per) fl |= FLUX_PLAIN;
-  return fl;
+  return per ? fl | flux_plain_bits(f.twod, f.fluxorder, f.weno_order) : fl;
 }
 
 static cudaError_t launch_stage(cb_ctx *c, const DevFields &F, int istage, double alfa, double beta, double adt, bool rhs_mode) {
@@ -621,24 +619,10 @@ int cb_create(const cb_config *cfg, cb_ctx **out) {
   }
   cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream);
   if (fill_ptab(c)) return bail(CB_E_CUDA, "pointer table");
-  // k-chunk: whole waves of the resident blocks (1 per SM in the FP64 form,
-  // 2 in the mixed form); a chunk's prologue costs about one plane.  Small
-  // blocks take chunks down to one plane: 32^3 FP64 44.2 us per stage at
-  // k-chunk 4, 30.2 at 2; mixed 30.7 at 4, 21.0 at 1.  The autotuner
-  // (cb_autotune) refines this by measurement.
   {
     const int by = cfg->weno_order == 5 ? SBY_W5 : BY;
-    const int tiles = ((cfg->mx - 2 + BX - 1) / BX) * ((cfg->my - 2 + by - 1) / by);
-    const int nk = cfg->mz - 2;
-    const int slots = c->sms * (cfg->precision == CB_MIXED ? 2 : 1);
-    double best = 1e30;
-    for (int kc = 1; kc <= nk; kc++) {
-      const int chunks = (nk + kc - 1) / kc;
-      const long long blocks = (long long)tiles * chunks;
-      const long long waves = (blocks + slots - 1) / slots;
-      const double cost = (double)waves * (kc + 1.0);
-      if (cost < best) { best = cost; c->kchunk = kc; }
-    }
+    const int cols = ((cfg->mx - 2 + BX - 1) / BX) * ((cfg->my - 2 + by - 1) / by);
+    c->kchunk = default_kchunk(cols, cfg->mz - 2, c->sms, cfg->precision == CB_MIXED, flux_bits(c), cfg->les != 0);
   }
   *out = c;
   return CB_OK;

@@ -182,10 +182,8 @@ static int batch_flux_bits(const cb_config &f) {
     if (f.s_x == 1.0) fl |= FLUX_SIGMA1;
     else if (f.s_x == 0.0) fl |= FLUX_SIGMA0;
   }
-  // block faces are interfaces (bctype 7): with no 2-D mode and MUSCL (or
-  // WENO5-JS, whose reconstruction the W5 bit selects) the PLAIN variants
-  if (f.twod == 0 && (f.fluxorder == 2 || f.weno_order == 5)) fl |= FLUX_PLAIN;
-  return fl;
+  // block faces are interfaces (bctype 7): the PLAIN variants
+  return fl | flux_plain_bits(f.twod, f.fluxorder, f.weno_order);
 }
 
 // -les 2, 3, ... (not 10): the dynamic model (Compute_Smagorinsky_Constant_1)
@@ -195,7 +193,7 @@ static bool batch_dynamic(const cb_config &f) { return f.les >= 2 && f.les != 10
 // the boundary-code branches the PLAIN variants fold away.
 static int batch_bits(const cb_batch *b) {
   const int fl = batch_flux_bits(b->cfg);
-  return b->nphys ? (fl & ~FLUX_PLAIN) : fl;
+  return b->nphys ? (fl & ~(FLUX_PLAIN | FLUX_W3)) : fl;
 }
 
 // every block's nvert is zero: the stage kernels' no-IBM variant

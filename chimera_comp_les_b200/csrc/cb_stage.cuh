@@ -63,9 +63,16 @@ struct TileShape {
 // blend weight of exactly 1 or 0, and WENO5-JS reconstruction.  FLUX_PLAIN
 // (no-IBM variants): every face of the block is periodic or an interface
 // (bctype 7 on all six sides), -twoD is 0, and without FLUX_W5 the
-// reconstruction is MUSCL (fluxorder 2) -- the options the host checked, as
-// compile-time constants, so the kernel carries no other branch of them.
-constexpr int FLUX_ROE = 1, FLUX_SIGMA1 = 2, FLUX_SIGMA0 = 4, FLUX_W5 = 8, FLUX_PLAIN = 16;
+// reconstruction is MUSCL (fluxorder 2), or with FLUX_W3 the reference's WENO3
+// (fluxorder 3) -- the options the host checked, as compile-time constants, so
+// the kernel carries no other branch of them.
+constexpr int FLUX_ROE = 1, FLUX_SIGMA1 = 2, FLUX_SIGMA0 = 4, FLUX_W5 = 8, FLUX_PLAIN = 16, FLUX_W3 = 32;
+// the bits of a periodic or interface block's options (0: no PLAIN variant)
+inline int flux_plain_bits(int twod, int fluxorder, int weno_order) {
+  if (twod != 0) return 0;
+  if (weno_order == 5 || fluxorder == 2) return FLUX_PLAIN;
+  return fluxorder == 3 ? FLUX_PLAIN | FLUX_W3 : 0;
+}
 
 // Tile geometry of a stage-kernel variant.  The WENO3/MUSCL stencil reaches
 // one node beyond the face's two nodes: a ring of 4 planes (k-1 .. k+2) and a
@@ -583,7 +590,7 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
   if constexpr (!CEN_ONLY) {  // reconstruction and the upwind flux
     R QL[5], QR[5], pL, pR;
     constexpr bool PLAIN = (FLUX & FLUX_PLAIN) != 0;
-    const int fo = (PLAIN && !W5) ? 2 : c.fluxorder;
+    const int fo = (PLAIN && !W5) ? ((FLUX & FLUX_W3) != 0 ? 3 : 2) : c.fluxorder;
     bool first;
     if (LES) {
       double nsum2 = (d == 2) ? nv0 + (NV0 ? 0.0 : ldg(F.nvert + gidx(c, 1, gj, gk + 1))) : nv0 + nv1;  // quirk rhs.c:4046
@@ -1556,7 +1563,8 @@ static StageKern stage_nv0_kernel_w(int fl) {
 // (static, like the kernels: each object's selector returns its own kernels)
 template <typename R, bool MIX, bool LES, bool VISC>
 static StageKern stage_nv0_kernel(int fl) {
-  switch (fl & (FLUX_W5 | FLUX_PLAIN)) {
+  switch (fl & (FLUX_W5 | FLUX_PLAIN | FLUX_W3)) {
+    case FLUX_PLAIN | FLUX_W3: return stage_nv0_kernel_w<R, MIX, LES, VISC, FLUX_PLAIN | FLUX_W3>(fl);
     case FLUX_W5: return stage_nv0_kernel_w<R, MIX, LES, VISC, FLUX_W5>(fl);
     case FLUX_PLAIN: return stage_nv0_kernel_w<R, MIX, LES, VISC, FLUX_PLAIN>(fl);
     case FLUX_W5 | FLUX_PLAIN: return stage_nv0_kernel_w<R, MIX, LES, VISC, FLUX_W5 | FLUX_PLAIN>(fl);
@@ -1592,7 +1600,7 @@ static cudaError_t stage_attrs() {
   for (int fl : {0, FLUX_ROE, FLUX_W5, FLUX_ROE | FLUX_W5})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(stage_gen_kernel<R, MIX, LES, VISC, RHSM>(fl), attr, (int)stage_smem_for<R, MIX>(fl, false));
   if constexpr (!RHSM) {  // the no-IBM variants of the time step
-    for (int w : {0, FLUX_W5, FLUX_PLAIN, FLUX_W5 | FLUX_PLAIN})
+    for (int w : {0, FLUX_W5, FLUX_PLAIN, FLUX_PLAIN | FLUX_W3, FLUX_W5 | FLUX_PLAIN})
       for (int fl = 0; fl < (LES ? 6 : 2) && e == cudaSuccess; fl++)
         e = cudaFuncSetAttribute(stage_nv0_kernel<R, MIX, LES, VISC>(w | fl), attr, (int)stage_smem_for<R, MIX>(w | fl, true));
   }

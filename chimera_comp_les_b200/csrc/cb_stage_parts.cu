@@ -90,7 +90,8 @@ BatchKern batched_nv0_w(int fl) {
 template <typename R, bool MIX, bool LES, bool VISC>
 BatchKern batched_kernel(int fl, bool nv0) {
   if (nv0) {
-    switch (fl & (FLUX_W5 | FLUX_PLAIN)) {
+    switch (fl & (FLUX_W5 | FLUX_PLAIN | FLUX_W3)) {
+      case FLUX_PLAIN | FLUX_W3: return batched_nv0_w<R, MIX, LES, VISC, FLUX_PLAIN | FLUX_W3>(fl);
       case FLUX_W5: return batched_nv0_w<R, MIX, LES, VISC, FLUX_W5>(fl);
       case FLUX_PLAIN: return batched_nv0_w<R, MIX, LES, VISC, FLUX_PLAIN>(fl);
       case FLUX_W5 | FLUX_PLAIN: return batched_nv0_w<R, MIX, LES, VISC, FLUX_W5 | FLUX_PLAIN>(fl);
@@ -111,7 +112,7 @@ cudaError_t batched_attrs() {
   for (int fl : {0, FLUX_ROE, FLUX_W5, FLUX_ROE | FLUX_W5})
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(batched_kernel<R, MIX, LES, VISC>(fl, false), attr, (int)stage_smem_for<R, MIX>(fl, false));
-  for (int w : {0, FLUX_W5, FLUX_PLAIN, FLUX_W5 | FLUX_PLAIN})
+  for (int w : {0, FLUX_W5, FLUX_PLAIN, FLUX_PLAIN | FLUX_W3, FLUX_W5 | FLUX_PLAIN})
     for (int fl = 0; fl < (LES ? 6 : 2) && e == cudaSuccess; fl++)
       e = cudaFuncSetAttribute(batched_kernel<R, MIX, LES, VISC>(w | fl, true), attr,
                                (int)stage_smem_for<R, MIX>(w | fl, true));
