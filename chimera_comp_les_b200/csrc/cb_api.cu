@@ -74,11 +74,13 @@ struct cb_ctx {
   unsigned *status = nullptr;
   bool fully_periodic = true;  // every face bctype 7: one fused periodic BC kernel
   bool nv0 = true;             // nvert is zero everywhere: the stage kernel's no-IBM variant
+  int2 *mask_planes = nullptr;  // per tile column: the planes a nonzero nvert reaches
   bool nvz = true;             // nvert is zero everywhere (the eddy viscosity reads no nvert)
   int cur = 0;                // buffer with the current Q (== Qold between steps)
   int uc = -1;                // buffer of the last CalcUCat state, -1: none
   bool have_grid = false, have_state = false;
   int kchunk = 16;
+  bool kchunk_tuned = false;  // set by cb_autotune
   GraphSlot graphs[3][4][2];  // [cur][uc + 1][p_carry]
   bool use_graphs = true;
   // immersed bodies: interpolation after the stages, then FormBCS(user, 0)
@@ -148,6 +150,8 @@ static DevFields fields_for(cb_ctx *c, int in, int old, int out) {
   F.cx = c->coorxy;
   F.cy = c->coorxy ? c->coorxy + c->plane : nullptr;
   F.ti = c->ti_dev;
+  F.mask_planes = c->nvz || c->cfg.visT ? nullptr : c->mask_planes;  // the no-IBM tiles carry no Sutherland law
+  F.all_clean = c->nvz && !c->cfg.visT;
   return F;
 }
 
@@ -164,6 +168,14 @@ static int flux_bits(const cb_ctx *c) {
   bool per = true;
   for (int s = 0; s < 6; s++) per = per && f.bctype[s] == 7;
   return per ? fl | flux_plain_bits(f.twod, f.fluxorder, f.weno_order) : fl;
+}
+
+// the k-chunk of the block's stage launches until cb_autotune measures one
+static void set_default_kchunk(cb_ctx *c) {
+  if (c->kchunk_tuned) return;
+  const int fl = flux_bits(c), by = stage_tile_rows(fl);
+  const int cols = ((c->cfg.mx - 2 + BX - 1) / BX) * ((c->cfg.my - 2 + by - 1) / by);
+  c->kchunk = default_kchunk(cols, c->cfg.mz - 2, c->sms, c->cfg.precision == CB_MIXED, fl, c->cfg.les != 0, !c->nvz);
 }
 
 static cudaError_t launch_stage(cb_ctx *c, const DevFields &F, int istage, double alfa, double beta, double adt, bool rhs_mode) {
@@ -620,9 +632,10 @@ int cb_create(const cb_config *cfg, cb_ctx **out) {
   cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream);
   if (fill_ptab(c)) return bail(CB_E_CUDA, "pointer table");
   {
-    const int by = cfg->weno_order == 5 ? SBY_W5 : BY;
+    const int by = stage_tile_rows(flux_bits(c));
     const int cols = ((cfg->mx - 2 + BX - 1) / BX) * ((cfg->my - 2 + by - 1) / by);
-    c->kchunk = default_kchunk(cols, cfg->mz - 2, c->sms, cfg->precision == CB_MIXED, flux_bits(c), cfg->les != 0);
+    if (cudaMalloc(&c->mask_planes, sizeof(int2) * cols) != cudaSuccess) return bail(CB_E_CUDA, "cudaMalloc mask planes");
+    set_default_kchunk(c);
   }
   *out = c;
   return CB_OK;
@@ -658,6 +671,7 @@ void cb_destroy(cb_ctx *c) {
   if (c->ptab) cudaFree(c->ptab);
   if (c->status) cudaFree(c->status);
   if (c->ti_dev) cudaFree(c->ti_dev);
+  if (c->mask_planes) cudaFree(c->mask_planes);
   if (c->coorxy) cudaFree(c->coorxy);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -785,11 +799,18 @@ int cb_set_nvert(cb_ctx *c, const double *nvert) {
   const int q = nvert_codes_exact(nvert, nn);
   bool zero = true;
   for (size_t t = 0; t < nn && zero; t++) zero = nvert[t] == 0.0;
+  if (!zero) {
+    const int by = stage_tile_rows(flux_bits(c)), tx = (c->dc.mx - 2 + BX - 1) / BX;
+    mask_planes_kernel<<<tx * ((c->dc.my - 2 + by - 1) / by), 256, 0, c->stream>>>(c->dc, c->nvert, tx, by,
+                                                                                    c->mask_planes);
+    CB_CUDA(c, cudaGetLastError());
+  }
   const bool nv0 = zero && !c->cfg.visT;  // the no-IBM variants carry no Sutherland law
   if (q != c->dc.nvq || nv0 != c->nv0 || zero != c->nvz) {
     c->dc.nvq = q;
     c->nv0 = nv0;
     c->nvz = zero;
+    set_default_kchunk(c);
     invalidate_graphs(c);  // the graphs carry the config and the kernel variant
   }
   return CB_OK;
@@ -1109,6 +1130,7 @@ int cb_autotune(cb_ctx *c, int ncand, const int *cand, double *ms_out, int *nout
   cudaEventDestroy(e1);
   if (nout) *nout = (int)cs.size();
   c->kchunk = bkc;
+  c->kchunk_tuned = true;
   if (best) *best = bkc;
   invalidate_graphs(c);  // the graphs carry the launch shape
   return CB_OK;

@@ -92,6 +92,12 @@ struct DevFields {
   // node coordinates x, y (the k-lo inflow codes 52 and 47 read them) and the
   // step index user->ti of the running step (code 47), or nullptr
   const double *cx, *cy;
+  // planes of each tile column whose stencils reach a nonzero nvert (see
+  // mask_planes_kernel): the single-block stage kernels run every other plane
+  // without nvert.  nullptr with all_clean 0: no such split; all_clean: nvert
+  // is zero everywhere
+  const int2 *mask_planes;
+  int all_clean;
   const int *ti;
 };
 

@@ -27,8 +27,10 @@ inline dim3 stage_grid(const DevCfg &c, int kchunk, int slots, int by = SBY) {
 // their own ends, so segments win only by a margin of 12 % in the model
 // (128^3 MUSCL 271 -> 261; 160^3 461 -> 484 stays chunked), and not at all
 // with WENO5-JS or with both fluxes of the blend on every face (192^3
-// WENO5-JS 2180 -> 2480, 128^3 blend 485 -> 503).
-inline int default_kchunk(int cols, int nk, int sms, bool mixed, int fl, bool les) {
+// WENO5-JS 2180 -> 2480, 128^3 blend 485 -> 503).  Nor with an immersed body
+// (masked): its planes cost more, and a segment cannot give them to another
+// CTA (sphere 96x96x128 FP64: segments 1698, k-chunk 13 1135).
+inline int default_kchunk(int cols, int nk, int sms, bool mixed, int fl, bool les, bool masked) {
   const long long slots = (long long)sms * (mixed ? 2 : 1);
   double best = 1e300;
   int bkc = nk;
@@ -39,7 +41,7 @@ inline int default_kchunk(int cols, int nk, int sms, bool mixed, int fl, bool le
   }
   const bool heavy = (fl & FLUX_W5) || (les && !(fl & (FLUX_SIGMA0 | FLUX_SIGMA1)));
   const double seg = (double)((cols * (long long)nk + slots - 1) / slots) + 2.0;
-  if (mixed ? (!heavy && 1.12 * seg <= best) : seg <= best) bkc = 0;
+  if (!masked && (mixed ? (!heavy && 1.12 * seg <= best) : seg <= best)) bkc = 0;
   return bkc;
 }
 inline int stage_tile_rows(int fl) { return (fl & FLUX_W5) ? SBY_W5 : SBY; }
@@ -49,8 +51,7 @@ inline int stage_tile_rows(int fl) { return (fl & FLUX_W5) ? SBY_W5 : SBY; }
 // contraction, the mixed form with it -- and once more for the batched work
 // queue, so the many template variants build in parallel.
 //
-// fl: FLUX bits (FLUX_ROE, FLUX_W5; the constant-sigma bits apply with nv0
-// only); nv0: nvert is zero everywhere, the variant without any nvert test
+// fl: FLUX bits; nv0: nvert is zero everywhere, the variant without any nvert test
 // (time step only); slots: CTAs of the balanced-segment shape (kchunk 0).
 template <typename R, bool MIX, bool LES>
 struct StageLaunch {

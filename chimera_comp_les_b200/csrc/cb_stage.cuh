@@ -1514,6 +1514,15 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
 // contiguous ranges, one per resident CTA; a CTA marches each column piece of
 // its range with its own prologue.  Every node gets the same arithmetic in
 // both shapes (a chunk start recomputes its first k-face from the same data).
+//
+// A kernel with nvert (NV0 false) runs the planes of a column that no nonzero
+// nvert reaches (F.mask_planes) through the no-IBM tile code, which gives the
+// same values: on a body in the flow most of the block is such planes, and the
+// nvert loads and tests cost 1.6-1.7 times the plane (sphere 96x96x128,
+// WENO5-JS + Roe: mixed 545 -> 442 us per stage, FP64 1579 -> 1131).  A run of fewer than MASK_MIN_RUN clean
+// planes beside dirty ones stays with them: a piece of its own costs a
+// prologue, about one plane.
+constexpr int MASK_MIN_RUN = 5;
 template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX = 0, bool NV0 = false>
 static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThreads<FLUX, MIX>::MIN_BLOCKS)
     stage_kernel(const DevCfg c, const DevFields F, int istage, double alfa, double beta, double adt, int kchunk) {
@@ -1534,11 +1543,49 @@ static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThread
   }
   while (s < e) {
     const int col = (int)(s / nk), k0 = (int)(s - (long long)col * nk);
-    const int k1 = (int)min((long long)nk, k0 + (e - s));
-    stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, NV0>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage, alfa,
-                                                      beta, adt, smem_d);
+    int k1 = (int)min((long long)nk, k0 + (e - s));
+    bool clean = NV0;
+    if constexpr (!NV0) {
+      int lo = 0, hi = nk;  // dirty planes lo .. hi - 1 of the column
+      if (F.mask_planes != nullptr) { const int2 d = F.mask_planes[col]; lo = d.x; hi = d.y; }
+      else if (F.all_clean) hi = 0;
+      lo = max(lo, k0);
+      hi = min(hi, k1);
+      if (lo >= hi) clean = true;
+      else if (lo - k0 >= MASK_MIN_RUN) { clean = true; k1 = lo; }
+      else if (k1 - hi >= MASK_MIN_RUN) k1 = hi;
+    }
+    if (clean)
+      stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, true>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage,
+                                                          alfa, beta, adt, smem_d);
+    else if constexpr (!NV0)
+      stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, false>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage,
+                                                           alfa, beta, adt, smem_d);
     s += k1 - k0;
   }
+}
+
+// The dirty planes of each tile column (a block per column): plane k (0-based
+// interior index) is dirty when a node the column's faces of that plane may
+// read has nvert != 0 -- within three nodes in every direction (the WENO5-JS
+// stencil of the outermost faces), or in the column's rows at i = 1 (the
+// zeta-face test, rhs.c:4046).  out[col] = (first, last + 1), empty as (0, 0).
+static __global__ void mask_planes_kernel(const DevCfg c, const double *nvert, int tiles_x, int by, int2 *out) {
+  const int col = blockIdx.x, i0 = 1 + (col % tiles_x) * SBX, j0 = 1 + (col / tiles_x) * by;
+  const int ia = max(-2, i0 - 3), ib = min(c.mx + 1, i0 + SBX + 2), ja = max(-2, j0 - 3), jb = min(c.my + 1, j0 + by + 2);
+  const int w = ib - ia + 2, rows = jb - ja + 1;  // one more column: the node i = 1 of the row
+  __shared__ int lo, hi;
+  if (threadIdx.x == 0) { lo = c.mz; hi = -1; }
+  __syncthreads();
+  const long long total = (long long)w * rows * c.pz;
+  for (long long t = threadIdx.x; t < total; t += blockDim.x) {
+    const int x = (int)(t % w), y = (int)((t / w) % rows), k = (int)(t / ((long long)w * rows)) - 2;
+    const int i = x == w - 1 ? 1 : ia + x;
+    if (nvert[gidx(c, i, ja + y, k)] != 0.0) { atomicMin(&lo, k); atomicMax(&hi, k); }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    out[col] = hi < lo ? make_int2(0, 0) : make_int2(max(0, lo - 1 - 3), min(c.mz - 2, hi - 1 + 3 + 1));
 }
 
 // The time-step kernel without nvert (NV0) for FLUX bits fl: Roe, with LES
@@ -1571,9 +1618,25 @@ static StageKern stage_nv0_kernel(int fl) {
     default: return stage_nv0_kernel_w<R, MIX, LES, VISC, 0>(fl);
   }
 }
-// The general (nvert-reading) kernel for the Roe and WENO5 bits of fl.
+// The general (nvert-reading) kernel for the Roe and WENO5 bits of fl and, in a
+// time step with LES, the constant-sigma ones (what the blend multiplies by
+// zero is not formed, as in the no-IBM variants).
 template <typename R, bool MIX, bool LES, bool VISC, bool RHSM>
 static StageKern stage_gen_kernel(int fl) {
+  if constexpr (LES && !RHSM) {
+    switch (fl & (FLUX_ROE | FLUX_W5 | FLUX_SIGMA0 | FLUX_SIGMA1)) {
+      case FLUX_SIGMA0: return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_SIGMA0>;
+      case FLUX_ROE | FLUX_SIGMA0: return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_ROE | FLUX_SIGMA0>;
+      case FLUX_W5 | FLUX_SIGMA0: return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_W5 | FLUX_SIGMA0>;
+      case FLUX_ROE | FLUX_W5 | FLUX_SIGMA0:
+        return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_ROE | FLUX_W5 | FLUX_SIGMA0>;
+      case FLUX_SIGMA1:
+      case FLUX_ROE | FLUX_SIGMA1: return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_SIGMA1>;
+      case FLUX_W5 | FLUX_SIGMA1:
+      case FLUX_ROE | FLUX_W5 | FLUX_SIGMA1: return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_W5 | FLUX_SIGMA1>;
+      default: break;
+    }
+  }
   switch (fl & (FLUX_ROE | FLUX_W5)) {
     case FLUX_ROE: return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_ROE>;
     case FLUX_W5: return stage_kernel<R, MIX, LES, VISC, RHSM, FLUX_W5>;
@@ -1589,16 +1652,19 @@ inline int stage_threads(int fl) {
 template <typename R, bool MIX>
 size_t stage_smem_for(int fl, bool nv0) {
   const bool w5 = (fl & FLUX_W5) != 0;
-  if (nv0) return w5 ? stage_smem<R, MIX, true, true>() : stage_smem<R, MIX, true, false>();
-  return w5 ? stage_smem<R, MIX, false, true>() : stage_smem<R, MIX, false, false>();
+  const size_t clean = w5 ? stage_smem<R, MIX, true, true>() : stage_smem<R, MIX, true, false>();
+  const size_t gen = w5 ? stage_smem<R, MIX, false, true>() : stage_smem<R, MIX, false, false>();
+  // a kernel with nvert runs both kinds of tile (the batched one only its own)
+  return nv0 ? clean : (clean > gen ? clean : gen);
 }
 // Opt every variant of one (LES, VISC, RHSM) into its dynamic shared memory.
 template <typename R, bool MIX, bool LES, bool VISC, bool RHSM>
 static cudaError_t stage_attrs() {
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
   cudaError_t e = cudaSuccess;
-  for (int fl : {0, FLUX_ROE, FLUX_W5, FLUX_ROE | FLUX_W5})
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(stage_gen_kernel<R, MIX, LES, VISC, RHSM>(fl), attr, (int)stage_smem_for<R, MIX>(fl, false));
+  for (int sg : {0, FLUX_SIGMA0, FLUX_SIGMA1})
+    for (int fl : {sg, sg | FLUX_ROE, sg | FLUX_W5, sg | FLUX_ROE | FLUX_W5})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(stage_gen_kernel<R, MIX, LES, VISC, RHSM>(fl), attr, (int)stage_smem_for<R, MIX>(fl, false));
   if constexpr (!RHSM) {  // the no-IBM variants of the time step
     for (int w : {0, FLUX_W5, FLUX_PLAIN, FLUX_PLAIN | FLUX_W3, FLUX_W5 | FLUX_PLAIN})
       for (int fl = 0; fl < (LES ? 6 : 2) && e == cudaSuccess; fl++)
