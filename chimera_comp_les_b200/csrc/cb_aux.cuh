@@ -5,6 +5,7 @@
 // by the host and every kernel uses a grid-stride loop.
 #pragma once
 #include "cb_common.cuh"
+#include "cb_div.cuh"
 
 namespace cb {
 
@@ -180,7 +181,7 @@ static __global__ void bc_face_kernel(const DevCfg c, DevFields F, int dir, doub
   else { na = c.mx; a0 = (bc[2] == 1) ? 1 : 0; nb = ((bc[3] == 1) ? c.my - 1 : c.my) - a0; }
   const long long total = (long long)na * nb;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int a = (int)(t % na), b = (int)(t / na);
+    const int b = (int)((unsigned)t / (unsigned)na), a = (int)((unsigned)t - (unsigned)b * (unsigned)na);
     if (dir == 0) {  // rhs.c:601-636: j = a, k = b
       long long n = gidx(c, 0, a, b);
       if (bc[0] == 3) {
@@ -409,7 +410,7 @@ static __global__ void bc_periodic_dir_kernel(const DevCfg c, DevFields F, int d
   const long long s = gstride(c, dir);
   const long long total = (long long)na * nb;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int a = (int)(t % na), b = (int)(t / na);
+    const int b = (int)((unsigned)t / (unsigned)na), a = (int)((unsigned)t - (unsigned)b * (unsigned)na);
     long long lo, hi;
     bool do_lo = true, do_hi = true;
     if (dir == 0) {
@@ -456,7 +457,7 @@ static __global__ void bc_periodic_dir_p_kernel(const DevCfg c, const double *ps
   const long long s = gstride(c, dir);
   const long long total = (long long)na * nb;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int a = (int)(t % na), b = (int)(t / na);
+    const int b = (int)((unsigned)t / (unsigned)na), a = (int)((unsigned)t - (unsigned)b * (unsigned)na);
     long long lo, hi;
     bool do_lo = true, do_hi = true;
     if (dir == 0) {
@@ -557,12 +558,12 @@ static __global__ void __launch_bounds__(EDDY_BX *EDDY_BY, 4)
     for (int e = tid; e < EDDY_PN; e += EDDY_BX * EDDY_BY) {
       double u0 = 0., u1 = 0., u2 = 0.;
       if (stv[e]) {
-        const double r = stq[0][e];
+        const Den<double> r(stq[0][e]);
         // lUcat x = 0 with -twoD 1 (rhs.c:1349), except where the dynamic
         // model rewrote it from the state (les.c:255)
-        u0 = (c.twod == 1 && stv[e] == 1) ? 0. : stq[1][e] / r;
-        u1 = stq[2][e] / r;
-        u2 = stq[3][e] / r;
+        u0 = (c.twod == 1 && stv[e] == 1) ? 0. : r(stq[1][e]);
+        u1 = r(stq[2][e]);
+        u2 = r(stq[3][e]);
       }
       us[s][0][e] = u0;
       us[s][1][e] = u1;
@@ -629,6 +630,8 @@ static __global__ void __launch_bounds__(EDDY_BX *EDDY_BY, 4)
     }
   }
 }
+// (32^3 FP64: 16.9 us per launch with chunks of at least four planes and a
+// quotient chain per node, 7.7 with chunks from one plane and cb_div.cuh)
 // k-chunk of the eddy-viscosity march: the fewest whole waves of resident
 // blocks, each chunk paying two extra velocity planes (cost = waves x
 // (chunk + 2)); the result does not depend on it
@@ -642,12 +645,11 @@ static inline int eddy_kchunk(const DevCfg &c, int sms) {
     resident = nb;
   }
   const int nk = c.mz - 2;
-  if (nk <= 4) return nk < 1 ? 1 : nk;
   const long long tiles = (long long)((c.mx - 2 + EDDY_BX - 1) / EDDY_BX) * ((c.my - 2 + EDDY_BY - 1) / EDDY_BY);
   const long long slots = (long long)(sms > 0 ? sms : 1) * resident;
   int best = nk;
   double bc = 1e300;
-  for (int kc = 4; kc <= nk; kc++) {
+  for (int kc = 1; kc <= nk; kc++) {
     const long long blocks = tiles * ((nk + kc - 1) / kc);
     const double cost = (double)((blocks + slots - 1) / slots) * (kc + 2);
     if (cost < bc) { bc = cost; best = kc; }
@@ -666,18 +668,18 @@ static inline dim3 eddy_grid(const DevCfg &c, int kchunk) {
 // curvature rule with y = z = min(y, z).  Boundary nodes keep (s_x, s_y, s_z).
 __device__ __forceinline__ double sensor_ri(double fR, double f0, double fL, double ks) {
   const double dfL = fL - f0, dfR = f0 - fR;
-  return (fabs(2 * dfL * dfR) + ks) / (dfL * dfL + dfR * dfR + ks);
+  return Den<double>(dfL * dfL + dfR * dfR + ks)(fabs(2 * dfL * dfR) + ks);
 }
 __device__ __forceinline__ double sensor_ramp(double fL, double f0, double fR, double fRR, double ks) {
   const double rL = sensor_ri(fL, f0, fR, ks), rR = sensor_ri(f0, fR, fRR, ks);
   const double r = (rR < rL) ? rR : rL;
   const double rd = 0.5;
   const double rmax = (rd < r) ? r : rd;
-  return 0.5 + 0.5 * tanh(3.0 * (r - rd) / rmax) / tanh(3.0);
+  return 0.5 + Den<double>(tanh(3.0))(0.5 * tanh(Den<double>(rmax)(3.0 * (r - rd))));
 }
 __device__ __forceinline__ double eos_node(const DevCfg &c, const double *const *q, long long n) {
   const double r = q[0][n];
-  return r != 0.0 ? (c.gamma - 1) * (q[4][n] - 0.5 * (q[1][n] * q[1][n] + q[2][n] * q[2][n] + q[3][n] * q[3][n]) / r)
+  return r != 0.0 ? (c.gamma - 1) * (q[4][n] - Den<double>(r)(0.5 * (q[1][n] * q[1][n] + q[2][n] * q[2][n] + q[3][n] * q[3][n])))
                   : 0.0;
 }
 __device__ __forceinline__ double pmin(double a, double b) { return (a < b) ? a : b; }
@@ -694,7 +696,9 @@ static __global__ void sigma_sensor_kernel(const DevCfg c, const double *const *
   const long long total = (long long)c.px * c.py * c.pz;
   const long long si = 1, sj = c.px, sk = (long long)c.px * c.py;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % c.px) - 2, j = (int)((t / c.px) % c.py) - 2, k = (int)(t / sk) - 2;
+    int i, j, k;
+    split3((unsigned)t, c.px, c.py, i, j, k);
+    i -= 2; j -= 2; k -= 2;
     double sx = c.s_x, sy = c.s_y, sz = c.s_z;
     if (i >= 1 && i <= c.mx - 2 && j >= 1 && j <= c.my - 2 && k >= 1 && k <= c.mz - 2) {
       const long long n = t;
@@ -725,7 +729,9 @@ static __global__ void sigma_filter_kernel(const DevCfg c, const double *const *
   const long long total = (long long)c.px * c.py * c.pz;
   const long long si = 1, sj = c.px, sk = (long long)c.px * c.py;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % c.px) - 2, j = (int)((t / c.px) % c.py) - 2, k = (int)(t / sk) - 2;
+    int i, j, k;
+    split3((unsigned)t, c.px, c.py, i, j, k);
+    i -= 2; j -= 2; k -= 2;
     const bool inner = i >= 1 && i <= c.mx - 2 && j >= 1 && j <= c.my - 2 && k >= 1 && k <= c.mz - 2;
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -742,7 +748,9 @@ static __global__ void sigma_post_kernel(const DevCfg c, const double *const *ls
   const long long total = (long long)c.px * c.py * c.pz;
   const long long sj = c.px, sk = (long long)c.px * c.py;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % c.px) - 2, j = (int)((t / c.px) % c.py) - 2, k = (int)(t / sk) - 2;
+    int i, j, k;
+    split3((unsigned)t, c.px, c.py, i, j, k);
+    i -= 2; j -= 2; k -= 2;
     double x = ls[0][t], y = ls[1][t], z = ls[2][t];
     if (i >= 1 && i <= c.mx - 2 && j >= 1 && j <= c.my - 2 && k >= 1 && k <= c.mz - 2) {
       const double *ly = ls[1], *lz = ls[2];
@@ -776,7 +784,8 @@ static __global__ void metrics_interior_kernel(const DevCfg c, const double *con
   const long long nx = c.mx, ny = c.my, nz = c.mz, total = nx * ny * nz;
   const long long si = 1, sj = c.px, sk = (long long)c.px * c.py;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / (nx * ny));
+    int i, j, k;
+    split3((unsigned)t, c.mx, c.my, i, j, k);
     const long long n = gidx(c, i, j, k);
     const bool ii = i > 0 && i < c.mx - 1, jj = j > 0 && j < c.my - 1, kk = k > 0 && k < c.mz - 1;
     double dc[3], de[3], dz[3];
@@ -820,7 +829,7 @@ static __global__ void metrics_boundary_kernel(const DevCfg c, double *const *me
   const int na = d == 0 ? c.my : c.mx, nb = d == 2 ? c.my : c.mz;  // the two transverse extents
   const long long total = (long long)na * nb;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int a = (int)(t % na), b = (int)(t / na);
+    const int b = (int)((unsigned)t / (unsigned)na), a = (int)((unsigned)t - (unsigned)b * (unsigned)na);
     int i, j, k;
     if (d == 0) { i = hi ? c.mx - 1 : 0; j = a; k = b; }
     else if (d == 1) { j = hi ? c.my - 1 : 0; i = a; k = b; }
@@ -842,7 +851,8 @@ static __global__ void metrics_boundary_kernel(const DevCfg c, double *const *me
 static __global__ void unpack_kernel(const DevCfg c, const double *__restrict__ aos, int nc, double *const *planes) {
   const long long total = (long long)c.mx * c.my * c.mz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % c.mx), j = (int)((t / c.mx) % c.my), k = (int)(t / ((long long)c.mx * c.my));
+    int i, j, k;
+    split3((unsigned)t, c.mx, c.my, i, j, k);
     const long long g = gidx(c, i, j, k);
     for (int q = 0; q < nc; q++) planes[q][g] = aos[t * nc + q];
   }
@@ -851,7 +861,8 @@ static __global__ void unpack_kernel(const DevCfg c, const double *__restrict__ 
 static __global__ void pack_kernel(const DevCfg c, const double *const *planes, int nc, double *__restrict__ aos) {
   const long long total = (long long)c.mx * c.my * c.mz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % c.mx), j = (int)((t / c.mx) % c.my), k = (int)(t / ((long long)c.mx * c.my));
+    int i, j, k;
+    split3((unsigned)t, c.mx, c.my, i, j, k);
     const long long g = gidx(c, i, j, k);
     for (int q = 0; q < nc; q++) aos[t * nc + q] = planes[q][g];
   }
@@ -861,7 +872,8 @@ static __global__ void pack_kernel(const DevCfg c, const double *const *planes, 
 static __global__ void eos_pack_kernel(const DevCfg c, const double *const *q, double *__restrict__ p) {
   const long long total = (long long)c.mx * c.my * c.mz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % c.mx), j = (int)((t / c.mx) % c.my), k = (int)(t / ((long long)c.mx * c.my));
+    int i, j, k;
+    split3((unsigned)t, c.mx, c.my, i, j, k);
     const long long g = gidx(c, i, j, k);
     const double r = q[0][g], ru = q[1][g], rv = q[2][g], rw = q[3][g], re = q[4][g];
     p[t] = (c.gamma - 1) * (re - 0.5 * (ru * ru + rv * rv + rw * rw) / r);
@@ -886,7 +898,9 @@ static __global__ void spectral_radius_kernel(const DevCfg c, const double *cons
   const long long nx = c.mx - 2, ny = c.my - 2, nz = c.mz - 2, total = nx * ny * nz;
   double lmax = 0.0;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int i = 1 + (int)(t % nx), j = 1 + (int)((t / nx) % ny), k = 1 + (int)(t / (nx * ny));
+    int i, j, k;
+    split3((unsigned)t, c.mx - 2, c.my - 2, i, j, k);
+    i++; j++; k++;
     const long long n = gidx(c, i, j, k);
     if (ldg(nvert + n) >= 0.1) continue;  // solid and interface nodes carry no RHS (rhs.c:4610)
     const double r = ldg(q[0] + n), u = ldg(q[1] + n) / r, v = ldg(q[2] + n) / r, w = ldg(q[3] + n) / r;

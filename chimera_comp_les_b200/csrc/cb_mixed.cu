@@ -16,7 +16,9 @@ __global__ void mixed_prep_kernel(const DevCfg c, const double *const *met, cons
     const float w[3] = {(float)delta2[t], (float)aj[t], 0.f};
     for (int e = 0; e < 3; e++)
       met4[e][t] = make_float4((float)met[3 * e][t], (float)met[3 * e + 1][t], (float)met[3 * e + 2][t], w[e]);
-    const int i = (int)(t % nx) - 2, j = (int)((t / nx) % ny) - 2, k = (int)(t / (nx * ny)) - 2;
+    int i, j, k;
+    split3((unsigned)t, c.px, c.py, i, j, k);
+    i -= 2; j -= 2; k -= 2;
     const bool interior = i >= 1 && i <= c.mx - 2 && j >= 1 && j <= c.my - 2 && k >= 1 && k <= c.mz - 2;
     for (int a = 0; a < 3; a++) {
       double s = 0.;
@@ -74,7 +76,7 @@ __global__ void __launch_bounds__(EF_BX *EF_BY)
     for (int e = tid; e < EF_PN; e += EF_BX * EF_BY) {
       float u0 = 0.f, u1 = 0.f, u2 = 0.f;
       if (stv[e]) {
-        const float ri = 1.f / (float)stq[0][e];
+        const float ri = rcp_approx((float)stq[0][e]);
         u0 = c.twod == 1 ? 0.f : (float)stq[1][e] * ri;  // lUcat x = 0 with -twoD 1 (rhs.c:1349)
         u1 = (float)stq[2][e] * ri;
         u2 = (float)stq[3][e] * ri;
@@ -151,12 +153,11 @@ int eddy_mixed_kchunk(const DevCfg &c, int sms) {
     resident = nb;
   }
   const int nk = c.mz - 2;
-  if (nk <= 4) return nk < 1 ? 1 : nk;
   const long long tiles = (long long)((c.mx - 2 + EF_BX - 1) / EF_BX) * ((c.my - 2 + EF_BY - 1) / EF_BY);
   const long long slots = (long long)(sms > 0 ? sms : 1) * resident;
   int best = nk;
   double bc = 1e300;
-  for (int kc = 4; kc <= nk; kc++) {  // the fewest whole waves, each chunk paying two extra planes
+  for (int kc = 1; kc <= nk; kc++) {  // the fewest whole waves, each chunk paying two extra planes
     const long long blocks = tiles * ((nk + kc - 1) / kc);
     const double cost = (double)((blocks + slots - 1) / slots) * (kc + 2);
     if (cost < bc) { bc = cost; best = kc; }
