@@ -24,6 +24,7 @@
 #include "cb_dyn.cuh"
 #include "cb_ibm.cuh"
 #include "cb_ibm_host.h"
+#include "cb_kchunk.h"
 #include "cb_launch.h"
 #include "cb_stage.cuh"
 
@@ -230,20 +231,18 @@ static void harvest_timing(cb_ctx *c) {
 }
 
 // Hybrid weights of the shock sensor from the stage input `in` (istage 0 of
-// formConvectionLES): three passes, each followed by the DMGlobalToLocal wrap.
+// formConvectionLES): three passes over every node of the padded box.  The
+// reference wraps the weights after each (DMGlobalToLocal); no pass and no face
+// reads one beyond the owned nodes, so the wraps are not formed here.
 // P: the pressure plane the first stage reads after an immersed step (lP
 // carried from the interpolation), else null (the EOS of the input).
 static int sigma_update(cb_ctx *c, int in, const double *P) {
   if (!c->dc.calc_sigma) return CB_OK;
   TimedScope ts(c, false);
   const int g = grid_for(c, (long long)c->plane);
-  const long long sh = shell_count(c->dc);
-  sigma_sensor_kernel<<<g, 256, 0, c->stream>>>(c->dc, (const double *const *)(c->ptab + 5 * in), c->ptab + PT_SIGA, P);
-  ghost_fill_kernel<<<grid_for(c, sh), 256, 0, c->stream>>>(c->dc, c->ptab + PT_SIGA, 3);
-  sigma_filter_kernel<<<g, 256, 0, c->stream>>>(c->dc, (const double *const *)(c->ptab + PT_SIGA), c->ptab + PT_SIGB);
-  ghost_fill_kernel<<<grid_for(c, sh), 256, 0, c->stream>>>(c->dc, c->ptab + PT_SIGB, 3);
-  sigma_post_kernel<<<g, 256, 0, c->stream>>>(c->dc, (const double *const *)(c->ptab + PT_SIGB), c->ptab + PT_SIGA);
-  ghost_fill_kernel<<<grid_for(c, sh), 256, 0, c->stream>>>(c->dc, c->ptab + PT_SIGA, 3);
+  launch_pdl(sigma_sensor_kernel, dim3(g), dim3(256), 0, c->stream, c->dc, (const double *const *)(c->ptab + 5 * in), c->ptab + PT_SIGA, P);
+  launch_pdl(sigma_filter_kernel, dim3(g), dim3(256), 0, c->stream, c->dc, (const double *const *)(c->ptab + PT_SIGA), c->ptab + PT_SIGB);
+  launch_pdl(sigma_post_kernel, dim3(g), dim3(256), 0, c->stream, c->dc, (const double *const *)(c->ptab + PT_SIGB), c->ptab + PT_SIGA);
   CB_CUDA(c, cudaGetLastError());
   return CB_OK;
 }
@@ -283,15 +282,11 @@ static int nut_update(cb_ctx *c) {
       CB_CUDA(c, launch_eddy_mixed(c->dc, qu, c->met4, c->nvz ? nullptr : c->nvert, c->nut, c->sms, c->stream));
     } else {
       const int ekc = eddy_kchunk(c->dc, c->sms);
-      eddy_viscosity_kernel<<<eddy_grid(c->dc, ekc), dim3(EDDY_BX, EDDY_BY), 0, c->stream>>>(
+      launch_pdl(eddy_viscosity_kernel, eddy_grid(c->dc, ekc), dim3(EDDY_BX, EDDY_BY), 0, c->stream, 
           c->dc, qu, (const double *const *)(c->ptab + PT_MET), c->aj, c->delta2, c->nvz ? nullptr : c->nvert, c->nut,
           ekc, dyn ? (const double *const *)(c->ptab + 5 * c->cur) : nullptr,
           dyn ? c->dyn_arena + 12 * c->plane : nullptr);
     }
-  }
-  {
-    TimedScope ts(c, false);
-    ghost_fill_kernel<<<grid_for(c, shell_count(c->dc)), 256, 0, c->stream>>>(c->dc, c->ptab + PT_NUT, 1);
   }
   CB_CUDA(c, cudaGetLastError());
   return CB_OK;
@@ -321,14 +316,14 @@ static int ibm_sweeps(cb_ctx *c, const IbmBody &b, int add_dundt, const double *
   const bool iso2 = c->cfg.isothermal == 2;
   const double a_sound = sqrt(c->cfg.twall / (c->cfg.ma * c->cfg.ma));  // ibm_iso.c:2768, the host's sqrt
   for (int s = 0; s < IBM_SWEEPS; s++) {
-    ibm_interp_kernel<<<g, 256, 0, c->stream>>>(c->dc, (const double *const *)(c->ptab + 5 * c->cur), c->pl, d,
+    launch_pdl(ibm_interp_kernel, dim3(g), dim3(256), 0, c->stream, c->dc, (const double *const *)(c->ptab + 5 * c->cur), c->pl, d,
                                                 add_dundt, c->ibm_twoD, slip, iso1, wf2, iso2 ? rho_old : nullptr,
                                                 a_sound);
     if (iso2) {
-      ibm_iso2_chain_kernel<<<1, IBM_CHAIN_NT, 0, c->stream>>>(c->dc, d, s == 0 ? 1 : 0, a_sound);
-      ibm_iso2_finish_kernel<<<g, 256, 0, c->stream>>>(c->dc, d, add_dundt);
+      launch_pdl(ibm_iso2_chain_kernel, dim3(1), dim3(IBM_CHAIN_NT), 0, c->stream, c->dc, d, s == 0 ? 1 : 0, a_sound);
+      launch_pdl(ibm_iso2_finish_kernel, dim3(g), dim3(256), 0, c->stream, c->dc, d, add_dundt);
     }
-    ibm_scatter_kernel<<<g, 256, 0, c->stream>>>(c->dc, c->ptab + 5 * c->cur, c->pl, d);
+    launch_pdl(ibm_scatter_kernel, dim3(g), dim3(256), 0, c->stream, c->dc, c->ptab + 5 * c->cur, c->pl, d);
   }
   CB_CUDA(c, cudaGetLastError());
   return CB_OK;
@@ -336,7 +331,7 @@ static int ibm_sweeps(cb_ctx *c, const IbmBody &b, int add_dundt, const double *
 
 // EqOfState of the current state into the pressure plane (solvers.c:279).
 static int eos_to_plane(cb_ctx *c) {
-  eos_plane_kernel<<<grid_for(c, (long long)c->plane), 256, 0, c->stream>>>(
+  launch_pdl(eos_plane_kernel, dim3(grid_for(c, (long long)c->plane)), dim3(256), 0, c->stream, 
       c->dc, (const double *const *)(c->ptab + 5 * c->cur), c->pl);
   CB_CUDA(c, cudaGetLastError());
   return CB_OK;
@@ -352,9 +347,9 @@ static int formbcs_zero(cb_ctx *c, int old) {
   // at most two nodes beyond the boundary layer, on either side
   if (std::min(c->dc.mx, std::min(c->dc.my, c->dc.mz)) >= 6) {
     const long long thick = thick_shell_count(c->dc, 5);
-    thick_shell_copy_kernel<<<grid_for(c, thick), 256, 0, c->stream>>>(
+    launch_pdl(thick_shell_copy_kernel, dim3(grid_for(c, thick)), dim3(256), 0, c->stream, 
         c->dc, 5, (const double *const *)(c->ptab + 5 * c->cur), c->ptab + PT_SNAP, 5);
-    thick_shell_copy_kernel<<<grid_for(c, thick), 256, 0, c->stream>>>(
+    launch_pdl(thick_shell_copy_kernel, dim3(grid_for(c, thick)), dim3(256), 0, c->stream, 
         c->dc, 5, (const double *const *)(c->ptab + PT_PL), c->ptab + PT_SNAP + 5, 1);
   } else {  // every node lies within five layers of a face
     CB_CUDA(c, cudaMemcpyAsync(c->spare, c->qb[c->cur][0], sizeof(double) * 5 * c->plane, cudaMemcpyDeviceToDevice,
@@ -366,18 +361,18 @@ static int formbcs_zero(cb_ctx *c, int old) {
   F.pin = c->psnap;
   const long long shell = shell_count(c->dc);
   if (c->fully_periodic) {
-    bc_periodic_kernel<<<grid_for(c, shell), 256, 0, c->stream>>>(c->dc, F);
-    bc_periodic_p_kernel<<<grid_for(c, shell), 256, 0, c->stream>>>(c->dc, c->psnap, c->pl);
+    launch_pdl(bc_periodic_kernel, dim3(grid_for(c, shell)), dim3(256), 0, c->stream, c->dc, F);
+    launch_pdl(bc_periodic_p_kernel, dim3(grid_for(c, shell)), dim3(256), 0, c->stream, c->dc, c->psnap, c->pl);
   } else {
     const long long face = (long long)std::max(c->dc.mx, c->dc.my) * std::max(c->dc.my, c->dc.mz);
-    for (int dir = 0; dir < 3; dir++) bc_face_kernel<<<grid_for(c, face), 256, 0, c->stream>>>(c->dc, F, dir, 0.0);
+    for (int dir = 0; dir < 3; dir++) launch_pdl(bc_face_kernel, dim3(grid_for(c, face)), dim3(256), 0, c->stream, c->dc, F, dir, 0.0);
     for (int dir = 0; dir < 3; dir++)
       if (c->dc.bctype[2 * dir] == 7) {
-        bc_periodic_dir_kernel<<<grid_for(c, face), 256, 0, c->stream>>>(c->dc, F, dir);
-        bc_periodic_dir_p_kernel<<<grid_for(c, face), 256, 0, c->stream>>>(c->dc, c->psnap, c->pl, dir);
+        launch_pdl(bc_periodic_dir_kernel, dim3(grid_for(c, face)), dim3(256), 0, c->stream, c->dc, F, dir);
+        launch_pdl(bc_periodic_dir_p_kernel, dim3(grid_for(c, face)), dim3(256), 0, c->stream, c->dc, c->psnap, c->pl, dir);
       }
-    ghost_fill_kernel<<<grid_for(c, shell), 256, 0, c->stream>>>(c->dc, c->ptab + 5 * c->cur, 5);
-    ghost_fill_kernel<<<grid_for(c, shell), 256, 0, c->stream>>>(c->dc, c->ptab + PT_PL, 1);
+    launch_pdl(ghost_fill_kernel, dim3(grid_for(c, shell)), dim3(256), 0, c->stream, c->dc, c->ptab + 5 * c->cur, 5);
+    launch_pdl(ghost_fill_kernel, dim3(grid_for(c, shell)), dim3(256), 0, c->stream, c->dc, c->ptab + PT_PL, 1);
   }
   CB_CUDA(c, cudaGetLastError());
   return CB_OK;
@@ -385,7 +380,7 @@ static int formbcs_zero(cb_ctx *c, int old) {
 
 // Enqueue one time step (no graph).
 static int enqueue_step(cb_ctx *c) {
-  if (c->dc.bctype[4] == 47) step_index_advance_kernel<<<1, 1, 0, c->stream>>>(c->ti_dev);
+  if (c->dc.bctype[4] == 47) launch_pdl(step_index_advance_kernel, dim3(1), dim3(1), 0, c->stream, c->ti_dev);
   if (c->cfg.les && c->cfg.les != 10 && !c->cfg.inviscid) {  // solvers.c:28
     int e = nut_update(c);
     if (e) return e;
@@ -413,16 +408,16 @@ static int enqueue_step(cb_ctx *c) {
     {
       TimedScope ts(c, false);
       if (c->fully_periodic) {
-        bc_periodic_kernel<<<grid_for(c, shell), 256, 0, c->stream>>>(c->dc, F);
+        launch_pdl(bc_periodic_kernel, dim3(grid_for(c, shell)), dim3(256), 0, c->stream, c->dc, F);
       } else {  // FormBCS with boundary codes (rhs.c:477-1227)
-        bc_combine_kernel<<<grid_for(c, shell), 256, 0, c->stream>>>(c->dc, F, s, alfa, beta, adt);
+        launch_pdl(bc_combine_kernel, dim3(grid_for(c, shell)), dim3(256), 0, c->stream, c->dc, F, s, alfa, beta, adt);
         const long long face = (long long)std::max(c->dc.mx, c->dc.my) * std::max(c->dc.my, c->dc.mz);
         for (int dir = 0; dir < 3; dir++)
-          bc_face_kernel<<<grid_for(c, face), 256, 0, c->stream>>>(c->dc, F, dir, alfa);
+          launch_pdl(bc_face_kernel, dim3(grid_for(c, face)), dim3(256), 0, c->stream, c->dc, F, dir, alfa);
         for (int dir = 0; dir < 3; dir++)
           if (c->dc.bctype[2 * dir] == 7)
-            bc_periodic_dir_kernel<<<grid_for(c, face), 256, 0, c->stream>>>(c->dc, F, dir);
-        ghost_fill_kernel<<<grid_for(c, shell), 256, 0, c->stream>>>(c->dc, c->ptab + 5 * out, 5);
+            launch_pdl(bc_periodic_dir_kernel, dim3(grid_for(c, face)), dim3(256), 0, c->stream, c->dc, F, dir);
+        launch_pdl(ghost_fill_kernel, dim3(grid_for(c, shell)), dim3(256), 0, c->stream, c->dc, c->ptab + 5 * out, 5);
       }
     }
     CB_CUDA(c, cudaGetLastError());
@@ -705,11 +700,11 @@ int cb_launches_per_step(const cb_ctx *c) {
   const bool box = f.i_homo_filter && f.j_homo_filter && f.k_homo_filter;
   int dyn = 0;  // the dynamic model's kernels
   if (les_dynamic(f) && !f.inviscid) {
-    dyn = (homo || f.les == 3) ? 6 : 9;
+    dyn = (homo || f.les == 3) ? 5 : 8;
     if (homo) dyn += 1 + (box ? 2 : (f.i_homo_filter ? 1 : 0));
   }
   const bool model = f.les && f.les != 10 && !f.inviscid;
-  return (model ? 2 : 0) + dyn + per_stage * c->cfg.fluxorder + (c->dc.calc_sigma ? 6 : 0) + ib;
+  return (model ? 1 : 0) + dyn + per_stage * c->cfg.fluxorder + (c->dc.calc_sigma ? 3 : 0) + ib;
 }
 
 static int upload_planes(cb_ctx *c, const double *host, int nc, int pt_first, bool pinned_hint) {

@@ -104,22 +104,43 @@ __host__ __device__ __forceinline__ void thick_shell_node(const DevCfg &c, int L
   k = (int)K - 2;
 }
 
+// dst[p][d] = src[p][s] for nplanes planes, five at a time with every load
+// ahead of the stores: a plane after the other, each store may alias the next
+// load, so a copy of five planes took five memory latencies one after another
+template <class S>
+__device__ __forceinline__ void copy_planes(S src, long long s, double *const *dst, long long d, int nplanes) {
+  for (int p0 = 0; p0 < nplanes; p0 += 5) {
+    const int n = nplanes - p0;
+    double v[5], *o[5];
+#pragma unroll
+    for (int p = 0; p < 5; p++) {
+      o[p] = p < n ? dst[p0 + p] : nullptr;
+      v[p] = p < n ? src[p0 + p][s] : 0.;
+    }
+#pragma unroll
+    for (int p = 0; p < 5; p++)
+      if (p < n) o[p][d] = v[p];
+  }
+}
+
 // Copy of the planes' nodes within L layers of the faces (the part of a state
 // FormBCS reads: periodic images two nodes across, face codes two nodes in).
 static __global__ void thick_shell_copy_kernel(const DevCfg c, int L, const double *const *src, double *const *dst,
                                                int nplanes) {
   const long long total = thick_shell_count(c, L);
+  pdl_wait();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
     thick_shell_node(c, L, t, i, j, k);
     const long long g = gidx(c, i, j, k);
-    for (int p = 0; p < nplanes; p++) dst[p][g] = src[p][g];
+    copy_planes(src, g, dst, g, nplanes);
   }
 }
 
 // Writes every non-interior node (boundary layer + both ghost layers) of qout.
 static __global__ void bc_periodic_kernel(const DevCfg c, DevFields F) {
   const long long total = shell_count(c);
+  pdl_wait();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
     shell_node(c, t, i, j, k);
@@ -127,8 +148,11 @@ static __global__ void bc_periodic_kernel(const DevCfg c, DevFields F) {
     bool from_in;
     bc_source(c, i, j, k, si, sj, sk, from_in);
     const long long g = gidx(c, i, j, k), s = gidx(c, si, sj, sk);
+    double v[5];
 #pragma unroll
-    for (int q = 0; q < 5; q++) F.qout[q][g] = from_in ? F.q[q][s] : F.qout[q][s];
+    for (int q = 0; q < 5; q++) v[q] = from_in ? F.q[q][s] : F.qout[q][s];
+#pragma unroll
+    for (int q = 0; q < 5; q++) F.qout[q][g] = v[q];
   }
 }
 
@@ -144,22 +168,30 @@ static __global__ void bc_periodic_kernel(const DevCfg c, DevFields F) {
 // (1) owned non-interior nodes: istage 0 Qold + adt*0, else beta Qold + adt*0 + alfa Qin
 static __global__ void bc_combine_kernel(const DevCfg c, DevFields F, int istage, double alfa, double beta, double adt) {
   const long long total = shell_count(c);
+  pdl_wait();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
     shell_node(c, t, i, j, k);
     if (i < 0 || i >= c.mx || j < 0 || j >= c.my || k < 0 || k >= c.mz) continue;
     const long long n = gidx(c, i, j, k);
+    double qo[5], qi[5];
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-      const double qo = F.qold[q][n];
-      F.qout[q][n] = (istage == 0) ? qo + adt * 0.0 : beta * qo + adt * 0.0 + alfa * F.q[q][n];
+      qo[q] = F.qold[q][n];
+      qi[q] = istage == 0 ? 0. : F.q[q][n];
     }
+#pragma unroll
+    for (int q = 0; q < 5; q++)
+      F.qout[q][n] = (istage == 0) ? qo[q] + adt * 0.0 : beta * qo[q] + adt * 0.0 + alfa * qi[q];
   }
 }
 
 // user->ti of the step about to run: the time loop advances it before
 // each step (main.c:887-974); the k-lo inflow code 47 reads it on the device
-static __global__ void step_index_advance_kernel(int *ti) { *ti += 1; }
+static __global__ void step_index_advance_kernel(int *ti) {
+  pdl_wait();
+  *ti += 1;
+}
 
 __device__ __forceinline__ double lp_at(const DevCfg &c, const DevFields &F, long long n) {
   if (F.pin) return F.pin[n];  // the pressure carried in lP
@@ -170,7 +202,15 @@ __device__ __forceinline__ double lp_at(const DevCfg &c, const DevFields &F, lon
 
 // (2) one direction's two faces; a thread per face node (lo and hi, as the
 // reference's loop body)
+struct Node5 {  // the five values of a node, loaded ahead of any store
+  double v[5];
+  __device__ __forceinline__ Node5(double *const *q, long long n) {
+#pragma unroll
+    for (int a = 0; a < 5; a++) v[a] = q[a][n];
+  }
+};
 static __global__ void bc_face_kernel(const DevCfg c, DevFields F, int dir, double alfa) {
+  pdl_wait();
   double *const *q = F.qout;
   const int *bc = c.bctype;
   const double g = c.gamma, Ma = c.ma;
@@ -185,22 +225,26 @@ static __global__ void bc_face_kernel(const DevCfg c, DevFields F, int dir, doub
     if (dir == 0) {  // rhs.c:601-636: j = a, k = b
       long long n = gidx(c, 0, a, b);
       if (bc[0] == 3) {
-        q[0][n] = q[0][n + si]; q[1][n] = 0.; q[2][n] = q[2][n + si]; q[3][n] = q[3][n + si]; q[4][n] = q[4][n + si];
+        const Node5 w(q, n + si);
+        q[0][n] = w.v[0]; q[1][n] = 0.; q[2][n] = w.v[2]; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[0] == 51) {
         q[0][n] = 0.445; q[1][n] = 0.311; q[2][n] = 0.; q[3][n] = 0.; q[4][n] = 8.928;
       }
       n = gidx(c, c.mx - 1, a, b);
       if (bc[1] == 3) {
-        q[0][n] = q[0][n - si]; q[1][n] = 0.; q[2][n] = q[2][n - si]; q[3][n] = q[3][n - si]; q[4][n] = q[4][n - si];
+        const Node5 w(q, n - si);
+        q[0][n] = w.v[0]; q[1][n] = 0.; q[2][n] = w.v[2]; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[0] == 51) {  // the high-i Lax state is keyed on bctype[0] (rhs.c:627)
         q[0][n] = 0.5; q[1][n] = 0.; q[2][n] = 0.; q[3][n] = 0.; q[4][n] = 1.4275;
       }
     } else if (dir == 1) {  // rhs.c:639-835: i = a, k = b
       long long n = gidx(c, a, 0, b);
       if (bc[2] == 3) {
-        q[0][n] = q[0][n + sj]; q[1][n] = q[1][n + sj]; q[2][n] = 0.; q[3][n] = q[3][n + sj]; q[4][n] = q[4][n + sj];
+        const Node5 w(q, n + sj);
+        q[0][n] = w.v[0]; q[1][n] = w.v[1]; q[2][n] = 0.; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[2] == 10) {
-        q[0][n] = q[0][n + sj]; q[1][n] = 0.; q[2][n] = q[2][n + sj]; q[3][n] = q[3][n + sj]; q[4][n] = q[4][n + sj];
+        const Node5 w(q, n + sj);
+        q[0][n] = w.v[0]; q[1][n] = 0.; q[2][n] = w.v[2]; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[2] == 1) {
         q[1][n] = 0.0; q[2][n] = 0.0; q[3][n] = 0.0;
         if (c.isothermal == 2 && alfa != 0 && F.nvert[n] < 1.5) {
@@ -231,9 +275,11 @@ static __global__ void bc_face_kernel(const DevCfg c, DevFields F, int dir, doub
       }
       n = gidx(c, a, c.my - 1, b);
       if (bc[3] == 3) {
-        q[0][n] = q[0][n - sj]; q[1][n] = q[1][n - sj]; q[2][n] = 0.; q[3][n] = q[3][n - sj]; q[4][n] = q[4][n - sj];
+        const Node5 w(q, n - sj);
+        q[0][n] = w.v[0]; q[1][n] = w.v[1]; q[2][n] = 0.; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[3] == 10) {
-        q[0][n] = q[0][n - sj]; q[1][n] = 0.; q[2][n] = q[2][n - sj]; q[3][n] = q[3][n - sj]; q[4][n] = q[4][n - sj];
+        const Node5 w(q, n - sj);
+        q[0][n] = w.v[0]; q[1][n] = 0.; q[2][n] = w.v[2]; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[3] == 1) {
         q[1][n] = 0.0; q[2][n] = 0.0; q[3][n] = 0.0;
         if (c.isothermal == 2) {  // rhs.c:803-818
@@ -259,12 +305,14 @@ static __global__ void bc_face_kernel(const DevCfg c, DevFields F, int dir, doub
       const int j = a0 + b;
       long long n = gidx(c, a, j, 0);
       if (bc[4] == 3) {
-        q[0][n] = q[0][n + sk]; q[1][n] = q[1][n + sk]; q[2][n] = q[2][n + sk]; q[3][n] = 0.; q[4][n] = q[4][n + sk];
+        const Node5 w(q, n + sk);
+        q[0][n] = w.v[0]; q[1][n] = w.v[1]; q[2][n] = w.v[2]; q[3][n] = 0.; q[4][n] = w.v[4];
       } else if (bc[4] == 55) {  // u = Ma, rho = gamma (rhs.c:837)
         const double rho = g, u = Ma;
         q[0][n] = rho; q[3][n] = rho * u; q[4][n] = 0.5 * rho * u * u + 1. / (g - 1.);
       } else if (bc[4] == 44) {
-        q[0][n] = q[0][n + sk]; q[1][n] = 0.; q[2][n] = 0.; q[3][n] = q[3][n + sk]; q[4][n] = q[4][n + sk];
+        const Node5 w(q, n + sk);
+        q[0][n] = w.v[0]; q[1][n] = 0.; q[2][n] = 0.; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[4] == 45) {
         q[0][n] = 1.; q[3][n] = 1.; q[4][n] = .5 + 1. / (Ma * Ma * g * (g - 1.));
       } else if (bc[4] == 51) {
@@ -324,11 +372,14 @@ static __global__ void bc_face_kernel(const DevCfg c, DevFields F, int dir, doub
       n = gidx(c, a, j, c.mz - 1);
       const long long m1 = n - sk, m2 = n - 2 * sk;
       if (bc[5] == 3) {
-        q[0][n] = q[0][m1]; q[1][n] = q[1][m1]; q[2][n] = q[2][m1]; q[3][n] = 0.; q[4][n] = q[4][m1];
+        const Node5 w(q, m1);
+        q[0][n] = w.v[0]; q[1][n] = w.v[1]; q[2][n] = w.v[2]; q[3][n] = 0.; q[4][n] = w.v[4];
       } else if (bc[5] == 44) {
-        q[0][n] = q[0][m1]; q[1][n] = 0.; q[2][n] = 0.; q[3][n] = q[3][m1]; q[4][n] = q[4][m1];
+        const Node5 w(q, m1);
+        q[0][n] = w.v[0]; q[1][n] = 0.; q[2][n] = 0.; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[5] == 45) {
-        q[0][n] = q[0][m1]; q[1][n] = q[1][m1]; q[2][n] = q[2][m1]; q[3][n] = q[3][m1]; q[4][n] = q[4][m1];
+        const Node5 w(q, m1);
+        q[0][n] = w.v[0]; q[1][n] = w.v[1]; q[2][n] = w.v[2]; q[3][n] = w.v[3]; q[4][n] = w.v[4];
       } else if (bc[5] == 49) {  // characteristic (rhs.c:1003-1042)
         double Vn, Rplus, Rminus, sv, pOverrho, pp;
         const double lp1 = lp_at(c, F, m1);
@@ -403,6 +454,7 @@ static __global__ void bc_face_kernel(const DevCfg c, DevFields F, int dir, doub
 // (i faces: 0 < k, 0 < j; j faces: j = 0 for k > 0, j = my-1 for 0 < k < mz-1;
 // k faces unguarded), from the stale ghosted stage input.
 static __global__ void bc_periodic_dir_kernel(const DevCfg c, DevFields F, int dir) {
+  pdl_wait();
   int na, nb;
   if (dir == 0) { na = c.my; nb = c.mz; }
   else if (dir == 1) { na = c.mx; nb = c.mz; }
@@ -423,10 +475,16 @@ static __global__ void bc_periodic_dir_kernel(const DevCfg c, DevFields F, int d
     } else {
       lo = gidx(c, a, b, 0); hi = gidx(c, a, b, c.mz - 1);
     }
+    double vl[5], vh[5];
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-      if (do_lo) F.qout[q][lo] = F.q[q][lo - 2 * s];
-      if (do_hi) F.qout[q][hi] = F.q[q][hi + 2 * s];
+      vl[q] = F.q[q][lo - 2 * s];
+      vh[q] = F.q[q][hi + 2 * s];
+    }
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+      if (do_lo) F.qout[q][lo] = vl[q];
+      if (do_hi) F.qout[q][hi] = vh[q];
     }
   }
 }
@@ -436,6 +494,7 @@ static __global__ void bc_periodic_dir_kernel(const DevCfg c, DevFields F, int d
 // `psnap` is P before the copies.
 static __global__ void bc_periodic_p_kernel(const DevCfg c, const double *psnap, double *P) {
   const long long total = shell_count(c);
+  pdl_wait();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
     shell_node(c, t, i, j, k);
@@ -450,6 +509,7 @@ static __global__ void bc_periodic_p_kernel(const DevCfg c, const double *psnap,
 // One periodic direction's pressure copies with the guards of
 // bc_periodic_dir_kernel.
 static __global__ void bc_periodic_dir_p_kernel(const DevCfg c, const double *psnap, double *P, int dir) {
+  pdl_wait();
   int na, nb;
   if (dir == 0) { na = c.my; nb = c.mz; }
   else if (dir == 1) { na = c.mx; nb = c.mz; }
@@ -478,6 +538,7 @@ static __global__ void bc_periodic_dir_p_kernel(const DevCfg c, const double *ps
 // EqOfState (rhs.c:4820-4862) on every node of the padded box; rho = 0
 // (unused padding) gives 0.
 static __global__ void eos_plane_kernel(const DevCfg c, const double *const *q, double *P) {
+  pdl_wait();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < c.plane; t += (long long)gridDim.x * blockDim.x) {
     const double r = q[0][t];
     P[t] = r != 0.0 ? (c.gamma - 1) * (q[4][t] - 0.5 * (q[1][t] * q[1][t] + q[2][t] * q[2][t] + q[3][t] * q[3][t]) / r)
@@ -488,6 +549,7 @@ static __global__ void eos_plane_kernel(const DevCfg c, const double *const *q, 
 // Ghost layers of periodic planes from their owned images (DMGlobalToLocal).
 static __global__ void ghost_fill_kernel(const DevCfg c, double *const *planes, int nplanes) {
   const long long total = shell_count(c);
+  pdl_wait();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int i, j, k;
     shell_node(c, t, i, j, k);
@@ -496,7 +558,7 @@ static __global__ void ghost_fill_kernel(const DevCfg c, double *const *planes, 
     const bool pi = c.bctype[0] == 7, pj = c.bctype[2] == 7, pk = c.bctype[4] == 7;
     if ((gi && !pi) || (gj && !pj) || (gk && !pk)) continue;
     const long long g = gidx(c, i, j, k), s = gidx(c, wrapi(i, c.mx), wrapi(j, c.my), wrapi(k, c.mz));
-    for (int p = 0; p < nplanes; p++) planes[p][g] = planes[p][s];
+    copy_planes(planes, s, planes, g, nplanes);
   }
 }
 
@@ -520,6 +582,7 @@ static __global__ void __launch_bounds__(EDDY_BX *EDDY_BY, 4)
   __shared__ double us[3][3][EDDY_PN];  // [slot][component][node]
   __shared__ double stq[4][EDDY_PN];    // raw rho, rhoU, rhoV, rhoW of the plane in flight
   __shared__ unsigned char stv[EDDY_PN];  // the staged node's velocity source: 0 none, 1 qu, 2 qn
+  pdl_wait();
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * EDDY_BX + tx;
   const int i0 = 1 + blockIdx.x * EDDY_BX, j0 = 1 + blockIdx.y * EDDY_BY;
   const int kb = 1 + blockIdx.z * kchunk, ke = min(c.mz - 1, kb + kchunk);
@@ -693,6 +756,7 @@ __device__ __forceinline__ double sensor_p(const DevCfg &c, const double *const 
 }
 static __global__ void sigma_sensor_kernel(const DevCfg c, const double *const *q, double *const *sig,
                                            const double *P) {
+  pdl_wait();
   const long long total = (long long)c.px * c.py * c.pz;
   const long long si = 1, sj = c.px, sk = (long long)c.px * c.py;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -726,6 +790,7 @@ static __global__ void sigma_sensor_kernel(const DevCfg c, const double *const *
 // pass 2 (ls: ghosted pass-1 planes): interior nodes times
 // sqrt(ls[j-1] ls) sqrt(ls[k-1] ls[k+1]) sqrt(ls[i-1] ls[i+1]); others copied
 static __global__ void sigma_filter_kernel(const DevCfg c, const double *const *ls, double *const *sig) {
+  pdl_wait();
   const long long total = (long long)c.px * c.py * c.pz;
   const long long si = 1, sj = c.px, sk = (long long)c.px * c.py;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -745,6 +810,7 @@ static __global__ void sigma_filter_kernel(const DevCfg c, const double *const *
 
 // pass 3 (ls: ghosted pass-2 planes): curvature rule, then y = z = min(z, y)
 static __global__ void sigma_post_kernel(const DevCfg c, const double *const *ls, double *const *sig) {
+  pdl_wait();
   const long long total = (long long)c.px * c.py * c.pz;
   const long long sj = c.px, sk = (long long)c.px * c.py;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {

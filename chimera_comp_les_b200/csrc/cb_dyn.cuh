@@ -496,7 +496,7 @@ static cudaError_t dyn_cs_enqueue(const DevCfg &dc, const DynOpts &o, const doub
     dyn_lm_tiled_kernel<<<grid, dim3(DYN_BX, DYN_BY), DYN_LM_SMEM, st>>>(dc, q, qu, aj, nvert, (const double *const *)D,
                                                                           P.sabs, P.lm, P.mm, kc, o.tf_mult, pointwise ? 0 : 1);
   }
-  ghost_fill_kernel<<<dyn_grid(shell, sms), 256, 0, st>>>(dc, D + 10, 2);
+  // (the reference wraps LM and MM here; the means around interior nodes read owned nodes only)
   const long long owned = (long long)dc.mx * dc.my * dc.mz;
   dyn_cs_kernel<<<dyn_grid(owned, sms), 256, 0, st>>>(dc, nvert, P.lm, P.mm, P.cs, o.max_cs, pointwise ? 1 : 0,
                                                       homo ? 0 : 1);

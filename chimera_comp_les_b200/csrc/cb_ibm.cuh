@@ -94,6 +94,7 @@ static __device__ __noinline__ double wf_find_utau(double nu, double u, double y
 static __global__ void __launch_bounds__(256) ibm_interp_kernel(const DevCfg c, const double *const *q, const double *P,
                                                                  IbmDev b, int add_dundt, int twoD, int slip, int iso1,
                                                                  int wf2, const double *rho_old, double a_sound) {
+  pdl_wait();
   const int n = b.n;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int cell = b.node[e].w;
@@ -207,6 +208,7 @@ static __global__ void __launch_bounds__(256) ibm_interp_kernel(const DevCfg c, 
 constexpr int IBM_CHAIN_NT = 256;
 static __global__ void __launch_bounds__(IBM_CHAIN_NT) ibm_iso2_chain_kernel(const DevCfg c, IbmDev b, int first,
                                                                             double a_sound) {
+  pdl_wait();
   __shared__ double sp[IBM_CHAIN_NT], sc1[IBM_CHAIN_NT], sx[IBM_CHAIN_NT], sr[IBM_CHAIN_NT], st[IBM_CHAIN_NT];
   const int n = b.n;
   const double *S = b.iso;
@@ -248,6 +250,7 @@ static __global__ void __launch_bounds__(IBM_CHAIN_NT) ibm_iso2_chain_kernel(con
 
 // -isothermal 2: each entry's conserved values from the chain's rho and p.
 static __global__ void __launch_bounds__(256) ibm_iso2_finish_kernel(const DevCfg c, IbmDev b, int add_dundt) {
+  pdl_wait();
   const int n = b.n;
   const double *S = b.iso;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
@@ -269,6 +272,7 @@ static __global__ void __launch_bounds__(256) ibm_iso2_finish_kernel(const DevCf
 // image of it in the periodic directions (the DMGlobalToLocal of Q and P that
 // ends a sweep).
 static __global__ void __launch_bounds__(256) ibm_scatter_kernel(const DevCfg c, double *const *q, double *P, IbmDev b) {
+  pdl_wait();
   const int n = b.n;
   const bool per[3] = {c.bctype[0] == 7, c.bctype[2] == 7, c.bctype[4] == 7};
   const int m[3] = {c.mx, c.my, c.mz};

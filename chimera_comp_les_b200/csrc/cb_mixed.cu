@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(EF_BX *EF_BY)
   __shared__ float us[3][3][EF_PN];       // [slot][component][node]
   __shared__ double stq[4][EF_PN];        // raw rho, rhoU, rhoV, rhoW of the plane in flight
   __shared__ unsigned char stv[EF_PN];    // the staged node has a velocity source
+  pdl_wait();
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * EF_BX + tx;
   const int i0 = 1 + blockIdx.x * EF_BX, j0 = 1 + blockIdx.y * EF_BY;
   const int kb = 1 + blockIdx.z * kchunk, ke = min(c.mz - 1, kb + kchunk);
@@ -171,8 +172,7 @@ cudaError_t launch_eddy_mixed(const DevCfg &c, const double *const *qu, const fl
   const int kc = eddy_mixed_kchunk(c, sms);
   const Met4 m4{{met4[0], met4[1], met4[2]}};
   const dim3 grid((c.mx - 2 + EF_BX - 1) / EF_BX, (c.my - 2 + EF_BY - 1) / EF_BY, (c.mz - 2 + kc - 1) / kc);
-  eddy_viscosity_mixed_kernel<<<grid, dim3(EF_BX, EF_BY), 0, s>>>(c, qu, m4, nvert, nut, kc);
-  return cudaGetLastError();
+  return launch_pdl(eddy_viscosity_mixed_kernel, grid, dim3(EF_BX, EF_BY), 0, s, c, qu, m4, nvert, nut, kc);
 }
 
 cudaError_t launch_mixed_prep(const DevCfg &c, const double *const *met, const double *delta2, const double *aj,

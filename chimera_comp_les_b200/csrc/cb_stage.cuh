@@ -1527,6 +1527,7 @@ template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX = 0
 static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThreads<FLUX, MIX>::MIN_BLOCKS)
     stage_kernel(const DevCfg c, const DevFields F, int istage, double alfa, double beta, double adt, int kchunk) {
   extern __shared__ double smem_d[];
+  pdl_wait();
   constexpr int BY = StageGeo<FLUX>::BY;
   const int nk = c.mz - 2, tiles_x = (c.mx - 2 + SBX - 1) / SBX;
   long long s, e;  // range of (column, plane) units, column-major

@@ -37,14 +37,14 @@ cudaError_t StageLaunch<R, MIX, LES>::attrs() {
 
 namespace {
 template <typename R, bool MIX, bool LES, bool VISC, bool RHSM>
-void launch_one(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta, double adt, int kchunk,
+cudaError_t launch_one(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta, double adt, int kchunk,
                 int fl, bool nv0, int slots, cudaStream_t s) {
   auto kern = stage_gen_kernel<R, MIX, LES, VISC, RHSM>(fl);
   const bool nv = !RHSM && nv0;
   if constexpr (!RHSM)
     if (nv0) kern = stage_nv0_kernel<R, MIX, LES, VISC>(fl);
-  kern<<<stage_grid(c, kchunk, slots, stage_tile_rows(fl)), stage_threads<MIX>(fl), stage_smem_for<R, MIX>(fl, nv), s>>>(
-      c, F, istage, alfa, beta, adt, kchunk);
+  return launch_pdl(kern, stage_grid(c, kchunk, slots, stage_tile_rows(fl)), dim3(stage_threads<MIX>(fl)),
+                    stage_smem_for<R, MIX>(fl, nv), s, c, F, istage, alfa, beta, adt, kchunk);
 }
 }  // namespace
 
@@ -53,13 +53,11 @@ cudaError_t StageLaunch<R, MIX, LES>::launch(const DevCfg &c, const DevFields &F
                                              double adt, int kchunk, bool visc, bool rhs_mode, int fl, bool nv0,
                                              int slots, cudaStream_t s) {
   if (rhs_mode) {
-    if (visc) launch_one<R, MIX, LES, true, true>(c, F, istage, alfa, beta, adt, kchunk, fl, false, slots, s);
-    else launch_one<R, MIX, LES, false, true>(c, F, istage, alfa, beta, adt, kchunk, fl, false, slots, s);
-  } else {
-    if (visc) launch_one<R, MIX, LES, true, false>(c, F, istage, alfa, beta, adt, kchunk, fl, nv0, slots, s);
-    else launch_one<R, MIX, LES, false, false>(c, F, istage, alfa, beta, adt, kchunk, fl, nv0, slots, s);
+    if (visc) return launch_one<R, MIX, LES, true, true>(c, F, istage, alfa, beta, adt, kchunk, fl, false, slots, s);
+    return launch_one<R, MIX, LES, false, true>(c, F, istage, alfa, beta, adt, kchunk, fl, false, slots, s);
   }
-  return cudaGetLastError();
+  if (visc) return launch_one<R, MIX, LES, true, false>(c, F, istage, alfa, beta, adt, kchunk, fl, nv0, slots, s);
+  return launch_one<R, MIX, LES, false, false>(c, F, istage, alfa, beta, adt, kchunk, fl, nv0, slots, s);
 }
 
 template struct StageLaunch<PartR, PART_MIX, PART_LES>;
