@@ -290,6 +290,46 @@ __device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
   return Den<R>(R(6.0) * ((a0 + a1) + a2))((a0 * q0 + a1 * q1) + a2 * q2);
 }
 
+// The mixed form's reconstructions of two fields at once.  The multiply-adds
+// are those the compiler forms from weno5 / weno3_l / weno3_r with FP32
+// contraction on (found by comparing every alternative bit for bit), so the
+// values are the scalar functions' own.
+__device__ __forceinline__ float2 weno5_2(float2 a, float2 b, float2 c, float2 d, float2 e) {
+  const float c13 = float(13.0 / 12.0);
+  const float2 eps = both(1e-6f), c2 = add2(c, c), c3 = mul2(3.f, c);
+  const float2 q0 = fma2(11.f, c, fma2(-7.f, b, add2(a, a)));
+  const float2 q1 = fma2(2.f, d, fma2(5.f, c, mul2(-1.f, b)));
+  const float2 q2 = sub2(fma2(5.f, d, c2), e);
+  const float2 t0 = add2(fma2(-2.f, b, a), c), u0 = add2(fma2(-4.f, b, a), c3);
+  const float2 t1 = add2(fma2(-2.f, c, b), d), u1 = sub2(b, d);
+  const float2 t2 = add2(fma2(-2.f, d, c), e), u2 = add2(fma2(-4.f, d, c3), e);
+  const float2 s0 = add2(eps, fma2(c13, mul2(t0, t0), mul2(0.25f, mul2(u0, u0))));
+  const float2 s1 = add2(eps, fma2(0.25f, mul2(u1, u1), mul2(c13, mul2(t1, t1))));
+  const float2 s2 = add2(eps, fma2(c13, mul2(t2, t2), mul2(0.25f, mul2(u2, u2))));
+  const float2 a0 = mul2(0.1f, rcp2(mul2(s0, s0)));
+  const float2 a1 = mul2(0.6f, rcp2(mul2(s1, s1)));
+  const float2 a2 = mul2(0.3f, rcp2(mul2(s2, s2)));
+  const float2 num = fma2(a2, q2, fma2(a0, q0, mul2(a1, q1)));
+  return mul2(num, rcp2(mul2(6.f, add2(add2(a0, a1), a2))));
+}
+// weno3_l(q0, q1, q2) and weno3_r(q1, q2, q3): both weigh the middle slope
+__device__ __forceinline__ void weno3_2(float2 q0, float2 q1, float2 q2, float2 q3, float2 &l, float2 &r) {
+  const float d0 = float(0.6666667), d1 = float(0.3333333);
+  const float2 eps = both(1e-6f), e0 = sub2(q0, q1), e1 = sub2(q2, q1), e2 = sub2(q3, q2);
+  const float2 s0 = fma2(e0, e0, eps), s1 = fma2(e1, e1, eps), s2 = fma2(e2, e2, eps);
+  const float2 y0 = rcp2(mul2(s0, s0)), y1 = rcp2(mul2(s1, s1)), y2 = rcp2(mul2(s2, s2));
+  {
+    const float2 a0 = mul2(d0, y1), a1 = mul2(d1, y0), y = rcp2(add2(a0, a1));
+    const float2 r0 = fma2(0.5f, q1, mul2(0.5f, q2)), r1 = fma2(1.5f, q1, mul2(-0.5f, q0));
+    l = fma2(mul2(a0, y), r0, mul2(mul2(a1, y), r1));
+  }
+  {
+    const float2 a0 = mul2(d0, y2), a1 = mul2(d1, y1), y = rcp2(add2(a0, a1));
+    const float2 r0 = fma2(1.5f, q2, mul2(-0.5f, q3)), r1 = fma2(0.5f, q1, mul2(0.5f, q2));
+    r = fma2(mul2(a0, y), r0, mul2(mul2(a1, y), r1));
+  }
+}
+
 // Conserved state and pressure of one node as the ring stores them, from its
 // raw FP64 state v (EqOfState rhs.c:4850; the mixed form shifts by the
 // reference state); pst/pin: the carried pressure of the FP64 form.  The
@@ -518,13 +558,26 @@ __device__ __forceinline__ bool weno5_face(const DevCfg &c, const DevFields &F, 
       node_qp<R, MIX>(c, v, pst, pst ? ldg(F.pin + g) : 0.0, qd, pd);
     }
   }
+  if constexpr (MIX) {  // fields two at a time; the pressure is the energy's partner
 #pragma unroll
-  for (int q = 0; q < 5; q++) {
-    QL[q] = weno5(Qm[q], Q[0][q], Q[1][q], Q[2][q], Q[3][q]);
-    QR[q] = weno5(Qp[q], Q[3][q], Q[2][q], Q[1][q], Q[0][q]);
+    for (int q = 0; q < 6; q += 2) {
+      auto pr = [&](const R *v, R p) { return make_float2(v[q], q == 4 ? p : v[q == 4 ? 4 : q + 1]); };
+      const float2 v0 = pr(Q[0], P[0]), v1 = pr(Q[1], P[1]), v2 = pr(Q[2], P[2]), v3 = pr(Q[3], P[3]);
+      const float2 l = weno5_2(pr(Qm, Pm), v0, v1, v2, v3), r = weno5_2(pr(Qp, Pp), v3, v2, v1, v0);
+      QL[q] = l.x;
+      QR[q] = r.x;
+      (q == 4 ? pL : QL[q == 4 ? 4 : q + 1]) = l.y;
+      (q == 4 ? pR : QR[q == 4 ? 4 : q + 1]) = r.y;
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+      QL[q] = weno5(Qm[q], Q[0][q], Q[1][q], Q[2][q], Q[3][q]);
+      QR[q] = weno5(Qp[q], Q[3][q], Q[2][q], Q[1][q], Q[0][q]);
+    }
+    pL = weno5(Pm, P[0], P[1], P[2], P[3]);
+    pR = weno5(Pp, P[3], P[2], P[1], P[0]);
   }
-  pL = weno5(Pm, P[0], P[1], P[2], P[3]);
-  pR = weno5(Pp, P[3], P[2], P[1], P[0]);
   return true;
 }
 
@@ -627,6 +680,25 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
       pR = muscl_r(P[1], P[2], wp ? P[1] : P[3]);
     } else if (W5 && weno5_face<R, MIX, NV0>(c, F, Rg, a, d, pos, m, g0, sd, Q, P, QL, QR, pL, pR)) {
       // WENO5-JS reconstruction of Q and p
+    } else if (MIX && NV0) {
+      if constexpr (MIX) {  // WENO3 without walls, fields two at a time
+#pragma unroll
+        for (int q = 0; q < 6; q += 2) {
+          auto pr = [&](int s) { return make_float2(Q[s][q], q == 4 ? P[s] : Q[s][q == 4 ? 4 : q + 1]); };
+          float2 l, r;
+          weno3_2(pr(0), pr(1), pr(2), pr(3), l, r);
+          QL[q] = l.x;
+          QR[q] = r.x;
+          (q == 4 ? pL : QL[q == 4 ? 4 : q + 1]) = l.y;
+          (q == 4 ? pR : QR[q == 4 ? 4 : q + 1]) = r.y;
+        }
+        if (!LES && !PLAIN && d == 1 && gj == 1 && c.isothermal && c.bctype[2] == 1) {  // rhs.c:2926
+          const int ord = c.eno_order;
+          QL[0] = eno_l(Q[1][0], Q[2][0], Q[3][0], ord);
+          QL[4] = eno_l(Q[1][4], Q[2][4], Q[3][4], ord);
+          pL = eno_l(P[1], P[2], P[3], ord);
+        }
+      }
     } else {
       const int ord = c.eno_order;
       const bool el = nvm > BLANKWALL && (d != 0 || (gi + 2) < c.mx);
