@@ -45,11 +45,12 @@ constexpr double GAMMA_CONV = 1.4;  // formConvection[LES] fix gamma = 1.4 (rhs.
 
 // face buffer width: FP64 keeps conv (5), visc (5), LES stress (3) apart to
 // difference them in the reference's order; the mixed form stores visc-conv.
-template <bool MIX>
+// Without viscous terms or without SGS terms (SgsTerms) those columns fall away.
+template <bool MIX, bool VISC = true, bool SGS = true>
 struct FaceWidth {
-  static constexpr int NG = MIX ? 8 : 13;
-  static constexpr int VOFF = MIX ? 0 : 5;   // visc offset
-  static constexpr int AOFF = MIX ? 5 : 10;  // LES stress offset
+  static constexpr int VOFF = MIX ? 0 : 5;                             // visc offset
+  static constexpr int AOFF = MIX ? 5 : (VISC ? 10 : 5);               // LES stress offset
+  static constexpr int NG = AOFF + (VISC && SGS ? 3 : 0);
 };
 
 template <int BX, int BY>
@@ -73,6 +74,15 @@ inline int flux_plain_bits(int twod, int fluxorder, int weno_order) {
   if (weno_order == 5 || fluxorder == 2) return FLUX_PLAIN;
   return fluxorder == 3 ? FLUX_PLAIN | FLUX_W3 : 0;
 }
+
+// Whether the viscous faces carry the LES stress (SGS viscosity and Yoshizawa
+// term) and the nodes its energy term: formViscous multiplies each of them by
+// sigma (rhs.c:1677-1710), so with the blend weight 0 on every face
+// (FLUX_SIGMA0) all of them are 0 for finite nu_t and are not formed, as the
+// central flux is not.  Per step: MUSCL 128^3 FP64 1.21 -> 1.05 ms, mixed 0.564
+// -> 0.518; WENO5-JS + Roe 192^3 mixed 5.52 -> 5.23; 96^3 FP64 1.95 -> 1.81.
+template <bool LES, bool VISC, int FLUX>
+constexpr bool SgsTerms = LES && VISC && (FLUX & FLUX_SIGMA0) == 0;
 
 // Tile geometry of a stage-kernel variant.  The WENO3/MUSCL stencil reaches
 // one node beyond the face's two nodes: a ring of 4 planes (k-1 .. k+2) and a
@@ -966,12 +976,12 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
           (g11 * dpdc + g21 * dpde + g31 * dpdz) * ajc * heat;
 
   A[0] = A[1] = A[2] = R(0.);
-  if (LES) {  // rhs.c:1677-1710
+  if constexpr (SgsTerms<LES, true, FLUX>) {  // rhs.c:1677-1710
     // the node weights: the constant the host chose the variant for, or sigma_at
-    constexpr bool S0 = (FLUX & FLUX_SIGMA0) != 0, S1 = (FLUX & FLUX_SIGMA1) != 0;
+    constexpr bool S1 = (FLUX & FLUX_SIGMA1) != 0;
     const int bi = gi + (d == 0), bj = gj + (d == 1), bk = gk + (d == 2);
-    const R sa = S0 ? R(0.) : (S1 ? R(1.) : R(sigma_at(c, F, d, gi, gj, gk)));
-    const R sb = S0 ? R(0.) : (S1 ? R(1.) : R(sigma_at(c, F, d, bi, bj, bk)));
+    const R sa = S1 ? R(1.) : R(sigma_at(c, F, d, gi, gj, gk));
+    const R sb = S1 ? R(1.) : R(sigma_at(c, F, d, bi, bj, bk));
     const double nu0 = SMET ? Rg.nut(a) : ldg(F.nut + g0);
     const double nu1 = (SMET && d < 2) ? Rg.nut(b) : ldg(F.nut + g1);
     R nut = R(0.5) * (R(nu0) * sa + R(nu1) * sb);
@@ -1008,7 +1018,8 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
 template <typename R, bool MIX, bool LES, bool VISC, class RG, int DIR, int FLUX = 0, bool NV0 = false>
 __device__ __forceinline__ void face_flux(const DevCfg &c, const DevFields &F, const RG &Rg, NRef a, int fi,
                                           int fj, int k, int drt, R *G) {
-  constexpr int VOFF = FaceWidth<MIX>::VOFF, AOFF = FaceWidth<MIX>::AOFF;
+  using W = FaceWidth<MIX, VISC, SgsTerms<LES, VISC, FLUX>>;
+  constexpr int VOFF = W::VOFF, AOFF = W::AOFF;
   R Fc[5], Fv[5], A[3];
   conv_face<R, MIX, LES, RG, DIR, FLUX, NV0>(c, F, Rg, a, fi, fj, k, drt, Fc);
   if (VISC) {
@@ -1023,9 +1034,9 @@ __device__ __forceinline__ void face_flux(const DevCfg &c, const DevFields &F, c
     for (int q = 0; q < 5; q++) G[q] = Fv[q] - Fc[q];
   } else {
 #pragma unroll
-    for (int q = 0; q < 5; q++) { G[q] = Fc[q]; G[VOFF + q] = Fv[q]; }
+    for (int q = 0; q < 5; q++) { G[q] = Fc[q]; if (VISC) G[VOFF + q] = Fv[q]; }
   }
-  G[AOFF] = A[0]; G[AOFF + 1] = A[1]; G[AOFF + 2] = A[2];
+  if constexpr (W::NG > AOFF) { G[AOFF] = A[0]; G[AOFF + 1] = A[1]; G[AOFF + 2] = A[2]; }
 }
 
 // The inviscid part (G[0..4]) or the viscous and SGS part (G[VOFF..VOFF+4],
@@ -1034,7 +1045,8 @@ __device__ __forceinline__ void face_flux(const DevCfg &c, const DevFields &F, c
 template <typename R, bool MIX, bool LES, bool VISC, class RG, int DIR, int FLUX = 0, bool NV0 = false>
 __device__ __forceinline__ void face_flux_half(const DevCfg &c, const DevFields &F, const RG &Rg, NRef a, int fi,
                                                int fj, int k, int drt, bool conv, R *G) {
-  constexpr int VOFF = FaceWidth<MIX>::VOFF, AOFF = FaceWidth<MIX>::AOFF;
+  using W = FaceWidth<MIX, VISC, SgsTerms<LES, VISC, FLUX>>;
+  constexpr int VOFF = W::VOFF, AOFF = W::AOFF;
   static_assert(!MIX, "the mixed form stores visc - conv per face");
   if (conv) {
     conv_face<R, MIX, LES, RG, DIR, FLUX, NV0>(c, F, Rg, a, fi, fj, k, drt, G);
@@ -1043,7 +1055,7 @@ __device__ __forceinline__ void face_flux_half(const DevCfg &c, const DevFields 
     visc_face<R, MIX, LES, RG, DIR, NV0, FLUX>(c, F, Rg, a, fi, fj, k, drt, Fv, A);
 #pragma unroll
     for (int q = 0; q < 5; q++) G[VOFF + q] = Fv[q];
-    G[AOFF] = A[0]; G[AOFF + 1] = A[1]; G[AOFF + 2] = A[2];
+    if constexpr (W::NG > AOFF) { G[AOFF] = A[0]; G[AOFF + 1] = A[1]; G[AOFF + 2] = A[2]; }
   }
 }
 
@@ -1148,8 +1160,8 @@ template <typename R, bool MIX, bool LES, bool VISC, bool ZONLY, int FLUX, bool 
 __device__ __forceinline__ void plane_faces(const DevCfg &c, const DevFields &F, const RG &Rg, int i0, int j0, int k,
                                             R *gxb, R *gyb, R *gzb, R *gzr) {
   using G = StageGeo<FLUX>;
-  constexpr int NT = G::NT, NG = FaceWidth<MIX>::NG;
-  constexpr int VOFF = FaceWidth<MIX>::VOFF;
+  using W = FaceWidth<MIX, VISC, SgsTerms<LES, VISC, FLUX>>;
+  constexpr int NT = G::NT, NG = W::NG, VOFF = W::VOFF;
   const int tid = threadIdx.x;
   if constexpr (StageThreads<FLUX, MIX>::SPLIT) {
     const int role = tid / NT;  // the half of the block (warp-uniform: NT is a multiple of 32)
@@ -1233,7 +1245,9 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
   constexpr int BX = G::BX, BY = G::BY, NPL = G::NPL, H = G::H;
   constexpr int NT = StageThreads<FLUX, MIX>::N;  // threads of the block
   constexpr int PX = G::Tile::PX, PN = G::Tile::PN, NXF = G::NXF, NYF = G::NYF, NZF = G::NZF;
-  constexpr int NG = FaceWidth<MIX>::NG, VOFF = FaceWidth<MIX>::VOFF, AOFF = FaceWidth<MIX>::AOFF;
+  constexpr bool SGS = SgsTerms<LES, VISC, FLUX>;
+  using FW = FaceWidth<MIX, VISC, SGS>;
+  constexpr int NG = FW::NG, VOFF = FW::VOFF, AOFF = FW::AOFF;
   constexpr int NSTG = StageSmem<R, MIX, NV0, G::W5>::NSTG;
   using RG = Ring<R, BX, BY, NPL>;
   constexpr bool SMET = StageMet<MIX, NV0, FLUX>::on;
@@ -1250,7 +1264,9 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
   R *gxb = smem + (size_t)NPL * NF * PN;  // [NG][NXF]
   R *gyb = gxb + (size_t)NG * NXF;        // [NG][NYF]
   R *gzb = gyb + (size_t)NG * NYF;        // [NG][NZF] (not with the metric slot)
-  unsigned char *nvc = reinterpret_cast<unsigned char *>(gzb + (SMET ? 0 : (size_t)NG * NZF));  // [NPL][PN]
+  // the face buffers' room (StageSmem sizes it for the widest variant), then [NPL][PN] nvert bytes
+  constexpr size_t FACES = (size_t)StageSmem<R, MIX, NV0, G::W5>::NG * (NXF + NYF + (SMET ? 0 : NZF));
+  unsigned char *nvc = reinterpret_cast<unsigned char *>(gxb + FACES);
   Rg.nvc = nvc;
   // staged fields per plane: Q, then nvert (byte-exact codes), then lP (carried pressure)
   const bool pst = !MIX && F.pin != nullptr;
@@ -1359,7 +1375,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
         const long long go = ok ? gidx(c, xi, yj, kk) : 0;  // src-size 0 below: nothing is read
 #pragma unroll
         for (int e = 0; e < 3; e++) cp_async16(mts + e * MPN + idx, F.met4[e] + go, ok);
-        if (LES) cp_async8(nts + idx, F.nut + go, ok);
+        if (SGS) cp_async8(nts + idx, F.nut + go, ok);
       }
       cp_async_commit();
     }
@@ -1375,8 +1391,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
   // at k-chunk 7, 32^3 FP64 30.2 -> 27.0 us at k-chunk 2).
   constexpr int NTB = StageThreads<FLUX, MIX>::N;
   double *aux = reinterpret_cast<double *>(gxb);  // [NPL][2][PN]: nvert, lP
-  static_assert(sizeof(R) * NG * (size_t)(NXF + NYF + (SMET ? 0 : NZF)) >=
-                    sizeof(double) * (size_t)PN * ((size_t)NPL * (NV0 ? 0 : 1) + (MIX ? 0 : NPL)),
+  static_assert(sizeof(R) * FACES >= sizeof(double) * (size_t)PN * ((size_t)NPL * (NV0 ? 0 : 1) + (MIX ? 0 : NPL)),
                 "the face buffers hold the prologue's nvert and lP planes");
   constexpr int AUXP = NV0 ? 0 : NPL * PN;  // first lP plane
   constexpr int RS = RG::AOS ? 1 : PN;      // stride of a node's raw doubles in the ring
@@ -1430,7 +1445,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
         const long long g1 = gidx(c, i0 + fx, j0 + fy, k + 1);
 #pragma unroll
         for (int e = 0; e < 3; e++) prefetch_l1(F.met4[e] + g1);
-        if (LES) prefetch_l1(F.nut + g1);
+        if (SGS) prefetch_l1(F.nut + g1);
       }
     }
     if constexpr (MIX) {
@@ -1453,7 +1468,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
     plane_faces<R, MIX, LES, VISC, false, FLUX, NV0>(c, F, Rg, i0, j0, k, gxb, gyb, gzb, gzr);
     // the only plane k-1 value the update needs, read before that slot is refilled
     const NRef n{0, uty + 2, utx + 2};
-    const R rho_km1 = (LES && VISC && uact) ? Rg.get(F_RHO, nshift(n, 2, -1)) : R(0.);
+    const R rho_km1 = (SGS && uact) ? Rg.get(F_RHO, nshift(n, 2, -1)) : R(0.);
     // the update's global operands, issued before the barrier so that their
     // latency overlaps the wait for the other warps' faces
     const long long g = gidx(c, ugi, ugj, k);
@@ -1504,6 +1519,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
         const R rD = (r0 + Rg.get(F_RHO, nshift(n, 1, -1))) * R(0.5), rU = (Rg.get(F_RHO, nshift(n, 1, 1)) + r0) * R(0.5);
         const R rB = (r0 + rho_km1) * R(0.5), rF = (Rg.get(F_RHO, nshift(n, 2, 1)) + r0) * R(0.5);
         R e = R(0.);
+        if constexpr (SGS) {
 #pragma unroll
         for (int q = 0; q < 3; q++) {
           const int a = AOFF + q;
@@ -1512,9 +1528,10 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
                       rF * (SMET ? gzr[a] : gzb[(size_t)a * NZF + fz]) - rB * Gzp[a];
           e = (q == 0) ? Rg.get(F_U + q, n) * t : e + Rg.get(F_U + q, n) * t;
         }
+        }
         return e;
       };
-      const bool les_e = LES && VISC && ugj > 2 && ugj < c.my - 2 && nv < 0.5;
+      const bool les_e = SGS && ugj > 2 && ugj < c.my - 2 && nv < 0.5;
       double rhs[5];
       if (MIX) {
         // G = visc - conv' (FP32); the p_ref * h part of conv is p_ref * gcl (FP64)
@@ -1536,7 +1553,10 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
         for (int q = 0; q < 5; q++) conv[q] = (nv < BLANK) ? fdiff(q) : R(0.);
         visc[0] = R(0.);
 #pragma unroll
-        for (int q = 1; q < 5; q++) visc[q] = VISC ? fdiff(VOFF + q) : R(0.);
+        for (int q = 1; q < 5; q++) {
+          if constexpr (VISC) visc[q] = fdiff(VOFF + q);
+          else visc[q] = R(0.);
+        }
         if (!PLAIN && c.twod == 1) conv[1] = visc[1] = R(0.);  // rhs.c:2135-2140, 3168-3173, 4215-4220
         if (LES && nv < BLANK && c.ratio != 0.0) {  // channel forcing (rhs.c:4226-4235); exact no-op at ratio 0
           const double ajn = aj_r;
