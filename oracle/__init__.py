@@ -469,13 +469,13 @@ class IbmSurface:
 
 # ------------------------------------------------------ shim-built reference --
 def ref_available() -> bool:
-    return os.path.exists(REF_SO) or os.path.isdir(REF_SRC_DIR)
+    return os.path.exists(REF_SO) or os.path.exists(os.path.join(REF_SRC_DIR, "rhs.c"))  # an empty folder is no checkout
 
 
 def build_ref(force: bool = False, optimized: bool = False, io: bool = False) -> str:
     so = REF_IO_SO if io else (REF_SO_O3 if optimized else REF_SO)
     if force or not os.path.exists(so):
-        if not os.path.isdir(REF_SRC_DIR):
+        if not os.path.exists(os.path.join(REF_SRC_DIR, "rhs.c")):
             raise FileNotFoundError("reference sources not present; cannot build oracle/_ref")
         subprocess.run(["make", "-s", "-C", _HERE, "ref", f"REF_DIR={REF_SRC_DIR}"], check=True)
     return so
