@@ -158,6 +158,17 @@ __device__ __forceinline__ MetV<R> met_load(const DevFields &F, int e, long long
   return r;
 }
 
+// Mean of two nodes' metric vectors (mixed form: two components per
+// instruction; w is the companion values' mean, FP64 form 0).
+__device__ __forceinline__ MetV<double> met_mean(const MetV<double> &a, const MetV<double> &b) {
+  return MetV<double>{0.5 * (a.x + b.x), 0.5 * (a.y + b.y), 0.5 * (a.z + b.z), 0.};
+}
+__device__ __forceinline__ MetV<float> met_mean(const MetV<float> &a, const MetV<float> &b) {
+  const float2 xy = mul2(0.5f, add2(make_float2(a.x, a.y), make_float2(b.x, b.y)));
+  const float2 zw = mul2(0.5f, add2(make_float2(a.z, a.w), make_float2(b.z, b.w)));
+  return MetV<float>{xy.x, xy.y, zw.x, zw.y};
+}
+
 __device__ __forceinline__ int bc_lo(const DevCfg &c, int d) { return d == 0 ? c.bctype[0] : (d == 1 ? c.bctype[2] : c.bctype[4]); }
 __device__ __forceinline__ int bc_hi(const DevCfg &c, int d) { return d == 0 ? c.bctype[1] : (d == 1 ? c.bctype[3] : c.bctype[5]); }
 
@@ -208,6 +219,11 @@ struct Ring {
       return pl[((slot(n.r) * NF + f) * PY + n.y) * PX + n.x];
     }
   }
+  // fields f, f + 1 (f even) of a node, mixed form
+  __device__ __forceinline__ float2 get2(int f, NRef n) const {
+    static_assert(AOS, "field pairs lie side by side in the mixed form's ring only");
+    return *reinterpret_cast<const float2 *>(pl + ((slot(n.r) * PY + n.y) * PX + n.x) * NF + f);
+  }
   __device__ __forceinline__ double nv(NRef n) const { return 0.25 * (double)nvc[(slot(n.r) * PY + n.y) * PX + n.x]; }
   // a node of the i/j halo rows the ring holds (the k range is always held)
   __device__ __forceinline__ bool holds(NRef n) const { return n.x >= 0 && n.x < PX && n.y >= 0 && n.y < PY; }
@@ -241,6 +257,10 @@ template <typename R>
 __device__ __forceinline__ R r_minmod(R a, R b) {
   const R m = copysign(fmin(fabs(a), fabs(b)), a);
   return (a * b < R(0)) ? R(0.) : m;
+}
+// FP32: the median of a, b and 0, the same value in one instruction less
+__device__ __forceinline__ float r_minmod(float a, float b) {
+  return fmaxf(fminf(a, b), fminf(fmaxf(a, b), 0.f));
 }
 template <typename R>
 __device__ __forceinline__ R muscl_l(R qm, R q0, R qp) { return q0 + R(0.5) * r_minmod(qp - q0, q0 - qm); }
@@ -298,6 +318,22 @@ __device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
   const R a1 = Den<R>((eps + b1) * (eps + b1))(R(0.6));
   const R a2 = Den<R>((eps + b2) * (eps + b2))(R(0.3));
   return Den<R>(R(6.0) * ((a0 + a1) + a2))((a0 * q0 + a1 * q1) + a2 * q2);
+}
+
+// The mixed form's MUSCL reconstruction of two fields at once:
+// muscl_l(q0, q1, q2) and muscl_r(q1, q2, q3), the scalar functions' values.
+// The kernel is bound by issue slots (61 % active): with this, the gradients and
+// the metric means in pairs a step of 128^3 MUSCL goes 0.518 -> 0.500 ms, 8
+// uneven WENO3 blocks (20 steps with transfers) 51.0 -> 49.7 ms, WENO5-JS + Roe
+// 192^3 5.23 -> 5.16 ms.  A pair operand that both lanes share costs a move, so
+// the products with one factor in common stay scalar.
+__device__ __forceinline__ float2 minmod2(float2 a, float2 b) {
+  return make_float2(r_minmod(a.x, b.x), r_minmod(a.y, b.y));
+}
+__device__ __forceinline__ void muscl_2(float2 q0, float2 q1, float2 q2, float2 q3, float2 &l, float2 &r) {
+  const float2 e0 = sub2(q1, q0), e1 = sub2(q2, q1), e2 = sub2(q3, q2);
+  l = fma2(0.5f, minmod2(e1, e0), q1);
+  r = fma2(-0.5f, minmod2(e2, e1), q2);
 }
 
 // The mixed form's reconstructions of two fields at once.  The multiply-adds
@@ -628,9 +664,12 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
     m1 = met_load<R, MIX>(F, d, g0 + sd);
   }
   R h[3];
-  h[0] = R(0.5) * (m0.x + m1.x);
-  h[1] = R(0.5) * (m0.y + m1.y);
-  h[2] = R(0.5) * (m0.z + m1.z);
+  {
+    const MetV<R> mm = met_mean(m0, m1);
+    h[0] = mm.x;
+    h[1] = mm.y;
+    h[2] = mm.z;
+  }
   const R pref = R(c.p_ref), href = R(c.h_ref);
 
   // stencil values along d: s=0..3 -> node offsets -1..2
@@ -679,15 +718,28 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
       for (int q = 0; q < 5; q++) { QL[q] = Q[1][q]; QR[q] = Q[2][q]; }
       pL = P[1]; pR = P[2];
     } else if (fo == 2 || (!LES && !W5 && d > 0 && gj < 30 && gk < 7)) {  // quirk rhs.c:2840, 2997
-      const bool wm = nvm > BLANKWALL;  // qm = q[i+1] when i-1 is a wall
-      const bool wp = nv2 > BLANKWALL;  // qp = q[i] when i+2 is a wall
-  #pragma unroll
-      for (int q = 0; q < 5; q++) {
-        QL[q] = muscl_l(wm ? Q[2][q] : Q[0][q], Q[1][q], Q[2][q]);
-        QR[q] = muscl_r(Q[1][q], Q[2][q], wp ? Q[1][q] : Q[3][q]);
+      if constexpr (MIX && NV0) {  // no walls: fields two at a time
+#pragma unroll
+        for (int q = 0; q < 6; q += 2) {
+          auto pr = [&](int s) { return make_float2(Q[s][q], q == 4 ? P[s] : Q[s][q == 4 ? 4 : q + 1]); };
+          float2 l, r;
+          muscl_2(pr(0), pr(1), pr(2), pr(3), l, r);
+          QL[q] = l.x;
+          QR[q] = r.x;
+          (q == 4 ? pL : QL[q == 4 ? 4 : q + 1]) = l.y;
+          (q == 4 ? pR : QR[q == 4 ? 4 : q + 1]) = r.y;
+        }
+      } else {
+        const bool wm = nvm > BLANKWALL;  // qm = q[i+1] when i-1 is a wall
+        const bool wp = nv2 > BLANKWALL;  // qp = q[i] when i+2 is a wall
+#pragma unroll
+        for (int q = 0; q < 5; q++) {
+          QL[q] = muscl_l(wm ? Q[2][q] : Q[0][q], Q[1][q], Q[2][q]);
+          QR[q] = muscl_r(Q[1][q], Q[2][q], wp ? Q[1][q] : Q[3][q]);
+        }
+        pL = muscl_l(wm ? P[2] : P[0], P[1], P[2]);
+        pR = muscl_r(P[1], P[2], wp ? P[1] : P[3]);
       }
-      pL = muscl_l(wm ? P[2] : P[0], P[1], P[2]);
-      pR = muscl_r(P[1], P[2], wp ? P[1] : P[3]);
     } else if (W5 && weno5_face<R, MIX, NV0>(c, F, Rg, a, d, pos, m, g0, sd, Q, P, QL, QR, pL, pR)) {
       // WENO5-JS reconstruction of Q and p
     } else if (MIX && NV0) {
@@ -840,6 +892,24 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
   const NRef b = nshift(a, d, 1);
   // D[f][e]: derivative of (u, v, w, T) along computational direction e
   R D[4][3];
+  if constexpr (MIX && NV0) {  // (u, v) and (w, T) in one instruction each
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+#pragma unroll
+      for (int f = 0; f < 4; f += 2) {
+        const int fi = F_U + f;
+        float2 t;
+        if (e == d) {
+          t = sub2(Rg.get2(fi, b), Rg.get2(fi, a));
+        } else {
+          const float2 p = add2(Rg.get2(fi, nshift(b, e, 1)), Rg.get2(fi, nshift(a, e, 1)));
+          t = mul2(0.25f, sub2(sub2(p, Rg.get2(fi, nshift(b, e, -1))), Rg.get2(fi, nshift(a, e, -1))));
+        }
+        D[f][e] = t.x;
+        D[f + 1][e] = t.y;
+      }
+    }
+  } else {
 #pragma unroll
   for (int e = 0; e < 3; e++) {
     if (e == d) {
@@ -868,6 +938,7 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
       }
     }
   }
+  }
   constexpr bool PLAIN = (FLUX & FLUX_PLAIN) != 0;
   if (!PLAIN && c.twod == 1) D[0][0] = D[0][1] = D[0][2] = R(0.);  // lUcat x = 0 (CalcUCat rhs.c:1349)
   const R dudc = D[0][0], dude = D[0][1], dudz = D[0][2];
@@ -876,7 +947,7 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
   const R dpdc = D[3][0], dpde = D[3][1], dpdz = D[3][2];
 
   R mh[3][3];
-  R w0[2], w1[2];  // mixed form: filter width and aj at g0 / g1
+  R w0 = R(0), ajm = R(0);  // mixed form: filter width at g0, mean aj
 #pragma unroll
   for (int e = 0; e < 3; e++) {
     MetV<R> p0, p1;
@@ -889,10 +960,12 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
       p0 = met_load<R, MIX>(F, e, g0);
       p1 = met_load<R, MIX>(F, e, g1);
     }
-    mh[e][0] = R(0.5) * (p0.x + p1.x);
-    mh[e][1] = R(0.5) * (p0.y + p1.y);
-    mh[e][2] = R(0.5) * (p0.z + p1.z);
-    if (e < 2) { w0[e] = p0.w; w1[e] = p1.w; }
+    const MetV<R> mm = met_mean(p0, p1);
+    mh[e][0] = mm.x;
+    mh[e][1] = mm.y;
+    mh[e][2] = mm.z;
+    if (e == 0) w0 = p0.w;
+    if (e == 1) ajm = mm.w;
   }
   const R md0 = d == 0 ? mh[0][0] : (d == 1 ? mh[1][0] : mh[2][0]);
   const R md1 = d == 0 ? mh[0][1] : (d == 1 ? mh[1][1] : mh[2][1]);
@@ -914,7 +987,7 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
   const R r23 = dvdc * csi2 + dvde * eta2 + dvdz * zet2;
   const R r33 = dwdc * csi2 + dwde * eta2 + dwdz * zet2;
 
-  const R ajc = MIX ? R(0.5) * (w0[1] + w1[1]) : R(0.5) * (R(ldg(F.aj + g0)) + R(ldg(F.aj + g1)));
+  const R ajc = MIX ? ajm : R(0.5) * (R(ldg(F.aj + g0)) + R(ldg(F.aj + g1)));
   R nu = R(c.inv_ren);  // 1./ren (evaluated once on the host, same value)
   if (LES) {
     // quirk: eta/zeta faces average rho over i and i+1 (rhs.c:1835, 2034)
@@ -991,7 +1064,7 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
     const R S2 = R(.5) * ((r11 - div) * (r11 - div) + r12 * r12 + r13 * r13 + r21 * r21 + (r22 - div) * (r22 - div) +
                           r23 * r23 + r31 * r31 + r32 * r32 + (r33 - div) * (r33 - div));
     // pow(pow(1/aj, 1/3), 2) of the left node, precomputed once per node
-    const R pf = MIX ? w0[0] : R(ldg(F.delta2 + g0));
+    const R pf = MIX ? w0 : R(ldg(F.delta2 + g0));
     if constexpr (MIX) {
       const R sn = ajc * (nut * rho_c);
       const R ks = -S2 * pf * R(c.ci * (2.0 / 3.0)) * (rho_c * sigma_c);
