@@ -1581,6 +1581,31 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
         prefetch_l2(F.aj + gu);
       }
     }
+    if constexpr (!MIX && (FLUX & FLUX_SIGMA1) != 0) {
+      // central flux alone: the metric planes of k+2 from DRAM into L2, a plane
+      // ahead of the first face that reads them.  These planes are the shortest
+      // of the FP64 form, too short for DRAM latency to hide (dynamic model
+      // 96x80x72 0.710 -> 0.682 ms per step); with an upwind flux the extra
+      // requests cost more (blend 0.829 -> 0.849, MUSCL 128^3 1.058 -> 1.069)
+      if (more) {
+        for (int idx = tid; idx < MPN; idx += NT) {
+          const int ly = idx / MPX, lx = idx - ly * MPX;
+          const int xi = i0 - 1 + lx, yj = j0 - 1 + ly;
+          if (xi <= c.mx + 1 && yj <= c.my + 1) {
+            const long long go = gidx(c, xi, yj, k + 2);  // k + 2 <= ke: inside the box
+#pragma unroll
+            for (int e = 0; e < 3; e++)
+#pragma unroll
+              for (int q = 0; q < 3; q++) prefetch_l2(F.met[e][q] + go);
+            prefetch_l2(F.aj + go);
+            if (SGS) {
+              prefetch_l2(F.nut + go);
+              prefetch_l2(F.delta2 + go);
+            }
+          }
+        }
+      }
+    }
     plane_faces<R, MIX, LES, VISC, false, FLUX, NV0>(c, F, Rg, i0, j0, k, gxb, gyb, gzb, gzr);
     // the only plane k-1 value the update needs, read before that slot is refilled
     const NRef n{0, uty + 2, utx + 2};
