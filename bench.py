@@ -71,8 +71,9 @@ def workload_config(n):
         "flux_variant": "sigma = 0 on every face (-s_x = -s_y = -s_z = 0, sensor off): the blend (1 - sigma) * "
                         "upwind + sigma * central equals the upwind flux, so the stage kernel forms only that; the "
                         "reference also multiplies the eddy viscosity and Yoshizawa terms by sigma, so the "
-                        "Smagorinsky model is inert in this flag set (its kernel still runs every step and the "
-                        "stage kernel still forms the SGS terms)",
+                        "Smagorinsky model is inert in this flag set (its kernel still runs every step; the "
+                        "stage kernel does not form the terms that sigma multiplies by zero, though the "
+                        "restatement's operation count in roofline.compute includes them)",
         "grid": [n + 2, n + 2, n + 2],
         "interior_nodes": n ** 3,
         "stages_per_step": CFG["fluxorder"],
