@@ -9,6 +9,8 @@ import glob
 import os
 import subprocess
 import sys
+import tempfile
+import time
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 REPO = os.path.dirname(PKG_DIR)
@@ -20,19 +22,20 @@ FP64_FLAGS = ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]
 MIXED_FLAGS = ["-fmad=true", "-prec-div=false", "-prec-sqrt=false"]
 _C = os.path.join(PKG_DIR, "csrc")
 # (source, flags, object name): cb_stage_parts.cu is compiled once per form
-# (FP64 / mixed), LES value and launch kind (single block / batched) so the
-# stage-kernel template variants build in parallel
+# (FP64 / mixed), LES and viscous value and launch kind (single block / batched)
+# so the stage-kernel template variants build in parallel, the longest first
 SOURCES = [
-    (os.path.join(_C, "cb_api.cu"), FP64_FLAGS, "cb_api"),
+    (os.path.join(_C, "cb_stage_parts.cu"),
+     (MIXED_FLAGS if mix else FP64_FLAGS)
+     + [f"-DCB_PART_MIX={mix}", f"-DCB_PART_LES={les}", f"-DCB_PART_VISC={visc}", f"-DCB_PART_BATCH={bat}"],
+     f"cb_stage_{'mixed' if mix else 'fp64'}_{'les' if les else 'std'}{'_visc' if visc else ''}{'_batch' if bat else ''}")
+    for les in (1, 0) for bat in (0, 1) for mix in (0, 1) for visc in (1, 0)
+] + [
     (os.path.join(_C, "cb_noalloc.cu"), FP64_FLAGS, "cb_noalloc"),
+    (os.path.join(_C, "cb_api.cu"), FP64_FLAGS, "cb_api"),
     (os.path.join(_C, "cb_batch.cu"), FP64_FLAGS, "cb_batch"),
     (os.path.join(_C, "cb_mixed.cu"), MIXED_FLAGS, "cb_mixed"),
     (os.path.join(_C, "cb_peaks.cu"), FP64_FLAGS, "cb_peaks"),
-] + [
-    (os.path.join(_C, "cb_stage_parts.cu"),
-     (MIXED_FLAGS if mix else FP64_FLAGS) + [f"-DCB_PART_MIX={mix}", f"-DCB_PART_LES={les}", f"-DCB_PART_BATCH={bat}"],
-     f"cb_stage_{'mixed' if mix else 'fp64'}_{'les' if les else 'std'}{'_batch' if bat else ''}")
-    for mix in (0, 1) for les in (1, 0) for bat in (0, 1)
 ]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NVCC_FLAGS = [
@@ -77,15 +80,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
     pending, running = list(cmds), []
     while pending or running:
         while pending and len(running) < jobs:
-            cmd = pending.pop(0)
-            running.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True)))
-        cmd, p = running.pop(0)
-        out, err = p.communicate()
-        if p.returncode != 0:
-            sys.stderr.write(out + err)
-            failed = failed or cmd
-        elif verbose:
-            sys.stderr.write(err)
+            cmd, log = pending.pop(0), tempfile.TemporaryFile("w+")
+            running.append((cmd, subprocess.Popen(cmd, stdout=log, stderr=log), log))
+        done = [r for r in running if r[1].poll() is not None]
+        if not done:
+            time.sleep(0.1)
+        for r in done:
+            running.remove(r)
+            cmd, p, log = r
+            log.seek(0)
+            if p.returncode != 0 or verbose:
+                sys.stderr.write(log.read())
+            if p.returncode != 0:
+                failed = failed or cmd
     if failed:
         raise RuntimeError("nvcc failed building libchimera_b200.so: " + " ".join(failed))
     _run([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB_PATH] + objs, verbose)

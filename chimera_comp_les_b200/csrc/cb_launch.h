@@ -18,69 +18,82 @@ inline dim3 stage_grid(const DevCfg &c, int kchunk, int slots, int by = SBY) {
 inline int stage_tile_rows(int fl) { return (fl & FLUX_W5) ? SBY_W5 : SBY; }
 
 // Launchers of the stage kernels, defined in cb_stage_parts.cu.  That file is
-// compiled once per (form, LES) pair -- the FP64 parity form without FMA
-// contraction, the mixed form with it -- and once more for the batched work
+// compiled once per (form, LES, viscous) triple -- the FP64 parity form without
+// FMA contraction, the mixed form with it -- and once more for the batched work
 // queue, so the many template variants build in parallel.
 //
 // fl: FLUX bits; nv0: nvert is zero everywhere, the variant without any nvert test
 // (time step only); slots: CTAs of the balanced-segment shape (kchunk 0).
-template <typename R, bool MIX, bool LES>
+template <typename R, bool MIX, bool LES, bool VISC>
 struct StageLaunch {
   static cudaError_t attrs();  // shared-memory opt-in of every variant
   static cudaError_t launch(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta, double adt,
-                            int kchunk, bool visc, bool rhs_mode, int fl, bool nv0, int slots, cudaStream_t s);
+                            int kchunk, bool rhs_mode, int fl, bool nv0, int slots, cudaStream_t s);
 };
 // The persistent multi-block work-queue launch (ctas CTAs).
-template <typename R, bool MIX, bool LES>
+template <typename R, bool MIX, bool LES, bool VISC>
 struct BatchLaunch {
   static cudaError_t attrs();
   static cudaError_t launch(const BatchBlock *tab, const int2 *items, int nitems, unsigned *counter, int istage,
-                            double alfa, double beta, double adt, bool visc, int fl, bool nv0, int ctas,
-                            cudaStream_t s);
+                            double alfa, double beta, double adt, int fl, bool nv0, int ctas, cudaStream_t s);
 };
 
-// Each (form, LES) instantiation is defined in exactly one object, the part
+// Each (form, LES, viscous) instantiation is defined in exactly one object, the part
 // built with that form's floating-point flags.  Without these declarations a
 // part would also instantiate the other parts' launchers (the inline
 // dispatchers below name all of them) and compile their kernels with its own
 // flags: an FP64 kernel built with FMA contraction, registered beside the
 // right one under the same host symbol.
-extern template struct StageLaunch<double, false, false>;
-extern template struct StageLaunch<double, false, true>;
-extern template struct StageLaunch<float, true, false>;
-extern template struct StageLaunch<float, true, true>;
-extern template struct BatchLaunch<double, false, false>;
-extern template struct BatchLaunch<double, false, true>;
-extern template struct BatchLaunch<float, true, false>;
-extern template struct BatchLaunch<float, true, true>;
+extern template struct StageLaunch<double, false, false, false>;
+extern template struct StageLaunch<double, false, false, true>;
+extern template struct StageLaunch<double, false, true, false>;
+extern template struct StageLaunch<double, false, true, true>;
+extern template struct StageLaunch<float, true, false, false>;
+extern template struct StageLaunch<float, true, false, true>;
+extern template struct StageLaunch<float, true, true, false>;
+extern template struct StageLaunch<float, true, true, true>;
+extern template struct BatchLaunch<double, false, false, false>;
+extern template struct BatchLaunch<double, false, false, true>;
+extern template struct BatchLaunch<double, false, true, false>;
+extern template struct BatchLaunch<double, false, true, true>;
+extern template struct BatchLaunch<float, true, false, false>;
+extern template struct BatchLaunch<float, true, false, true>;
+extern template struct BatchLaunch<float, true, true, false>;
+extern template struct BatchLaunch<float, true, true, true>;
 
-inline cudaError_t stage_attrs_all(bool mix) {
-  cudaError_t e = mix ? StageLaunch<float, true, true>::attrs() : StageLaunch<double, false, true>::attrs();
-  if (e == cudaSuccess) e = mix ? StageLaunch<float, true, false>::attrs() : StageLaunch<double, false, false>::attrs();
+// calls f with the launcher of a form, LES and viscous value
+template <template <typename, bool, bool, bool> class L, class Fn>
+inline cudaError_t with_part(bool mix, bool les, bool visc, Fn f) {
+  if (mix) {
+    if (les) return visc ? f(L<float, true, true, true>{}) : f(L<float, true, true, false>{});
+    return visc ? f(L<float, true, false, true>{}) : f(L<float, true, false, false>{});
+  }
+  if (les) return visc ? f(L<double, false, true, true>{}) : f(L<double, false, true, false>{});
+  return visc ? f(L<double, false, false, true>{}) : f(L<double, false, false, false>{});
+}
+template <template <typename, bool, bool, bool> class L>
+inline cudaError_t attrs_all(bool mix) {
+  cudaError_t e = cudaSuccess;
+  for (bool les : {true, false})
+    for (bool visc : {true, false})
+      if (e == cudaSuccess) e = with_part<L>(mix, les, visc, [](auto p) { return decltype(p)::attrs(); });
   return e;
 }
+inline cudaError_t stage_attrs_all(bool mix) { return attrs_all<StageLaunch>(mix); }
+inline cudaError_t batch_attrs_all(bool mix) { return attrs_all<BatchLaunch>(mix); }
 inline cudaError_t launch_stage_any(bool mix, bool les, const DevCfg &c, const DevFields &F, int istage, double alfa,
                                     double beta, double adt, int kchunk, bool visc, bool rhs_mode, int fl, bool nv0,
                                     int slots, cudaStream_t s) {
-  if (mix)
-    return les ? StageLaunch<float, true, true>::launch(c, F, istage, alfa, beta, adt, kchunk, visc, rhs_mode, fl, nv0, slots, s)
-               : StageLaunch<float, true, false>::launch(c, F, istage, alfa, beta, adt, kchunk, visc, rhs_mode, fl, nv0, slots, s);
-  return les ? StageLaunch<double, false, true>::launch(c, F, istage, alfa, beta, adt, kchunk, visc, rhs_mode, fl, nv0, slots, s)
-             : StageLaunch<double, false, false>::launch(c, F, istage, alfa, beta, adt, kchunk, visc, rhs_mode, fl, nv0, slots, s);
-}
-inline cudaError_t batch_attrs_all(bool mix) {
-  cudaError_t e = mix ? BatchLaunch<float, true, true>::attrs() : BatchLaunch<double, false, true>::attrs();
-  if (e == cudaSuccess) e = mix ? BatchLaunch<float, true, false>::attrs() : BatchLaunch<double, false, false>::attrs();
-  return e;
+  return with_part<StageLaunch>(mix, les, visc, [&](auto p) {
+    return decltype(p)::launch(c, F, istage, alfa, beta, adt, kchunk, rhs_mode, fl, nv0, slots, s);
+  });
 }
 inline cudaError_t launch_batched_any(bool mix, bool les, const BatchBlock *tab, const int2 *items, int nitems,
                                       unsigned *counter, int istage, double alfa, double beta, double adt, bool visc,
                                       int fl, bool nv0, int ctas, cudaStream_t s) {
-  if (mix)
-    return les ? BatchLaunch<float, true, true>::launch(tab, items, nitems, counter, istage, alfa, beta, adt, visc, fl, nv0, ctas, s)
-               : BatchLaunch<float, true, false>::launch(tab, items, nitems, counter, istage, alfa, beta, adt, visc, fl, nv0, ctas, s);
-  return les ? BatchLaunch<double, false, true>::launch(tab, items, nitems, counter, istage, alfa, beta, adt, visc, fl, nv0, ctas, s)
-             : BatchLaunch<double, false, false>::launch(tab, items, nitems, counter, istage, alfa, beta, adt, visc, fl, nv0, ctas, s);
+  return with_part<BatchLaunch>(mix, les, visc, [&](auto p) {
+    return decltype(p)::launch(tab, items, nitems, counter, istage, alfa, beta, adt, fl, nv0, ctas, s);
+  });
 }
 
 // FP32 metric vectors (w: filter width, aj, 0) and the FP64 metric divergence

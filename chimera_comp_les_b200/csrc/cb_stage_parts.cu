@@ -3,14 +3,15 @@
 //   CB_PART_MIX   0: FP64 parity form (built without FMA contraction, IEEE
 //                    division and square root), 1: mixed form (FMA, fast FP32)
 //   CB_PART_LES   the LES template value
+//   CB_PART_VISC  the viscous template value
 //   CB_PART_BATCH 0: single-block launches, 1: the batched work queue
 // The build compiles this file once per combination, so the template variants
-// (flux bits x viscous x no-IBM x RHS mode) compile in parallel.
+// (flux bits x no-IBM x RHS mode) compile in parallel.
 #include "cb_launch.h"
 #include "cb_stage.cuh"
 
 #ifndef CB_PART_MIX
-#error "compile with -DCB_PART_MIX=0|1 -DCB_PART_LES=0|1 -DCB_PART_BATCH=0|1"
+#error "compile with -DCB_PART_MIX=0|1 -DCB_PART_LES=0|1 -DCB_PART_VISC=0|1 -DCB_PART_BATCH=0|1"
 #endif
 
 namespace cb {
@@ -21,17 +22,15 @@ using PartR = float;
 #else
 using PartR = double;
 #endif
-constexpr bool PART_MIX = CB_PART_MIX != 0, PART_LES = CB_PART_LES != 0;
+constexpr bool PART_MIX = CB_PART_MIX != 0, PART_LES = CB_PART_LES != 0, PART_VISC = CB_PART_VISC != 0;
 }  // namespace
 
 #if !CB_PART_BATCH
 
-template <typename R, bool MIX, bool LES>
-cudaError_t StageLaunch<R, MIX, LES>::attrs() {
-  cudaError_t e = stage_attrs<R, MIX, LES, true, false>();
-  if (e == cudaSuccess) e = stage_attrs<R, MIX, LES, false, false>();
-  if (e == cudaSuccess) e = stage_attrs<R, MIX, LES, true, true>();
-  if (e == cudaSuccess) e = stage_attrs<R, MIX, LES, false, true>();
+template <typename R, bool MIX, bool LES, bool VISC>
+cudaError_t StageLaunch<R, MIX, LES, VISC>::attrs() {
+  cudaError_t e = stage_attrs<R, MIX, LES, VISC, false>();
+  if (e == cudaSuccess) e = stage_attrs<R, MIX, LES, VISC, true>();
   return e;
 }
 
@@ -48,19 +47,15 @@ cudaError_t launch_one(const DevCfg &c, const DevFields &F, int istage, double a
 }
 }  // namespace
 
-template <typename R, bool MIX, bool LES>
-cudaError_t StageLaunch<R, MIX, LES>::launch(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta,
-                                             double adt, int kchunk, bool visc, bool rhs_mode, int fl, bool nv0,
-                                             int slots, cudaStream_t s) {
-  if (rhs_mode) {
-    if (visc) return launch_one<R, MIX, LES, true, true>(c, F, istage, alfa, beta, adt, kchunk, fl, false, slots, s);
-    return launch_one<R, MIX, LES, false, true>(c, F, istage, alfa, beta, adt, kchunk, fl, false, slots, s);
-  }
-  if (visc) return launch_one<R, MIX, LES, true, false>(c, F, istage, alfa, beta, adt, kchunk, fl, nv0, slots, s);
-  return launch_one<R, MIX, LES, false, false>(c, F, istage, alfa, beta, adt, kchunk, fl, nv0, slots, s);
+template <typename R, bool MIX, bool LES, bool VISC>
+cudaError_t StageLaunch<R, MIX, LES, VISC>::launch(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta,
+                                                   double adt, int kchunk, bool rhs_mode, int fl, bool nv0, int slots,
+                                                   cudaStream_t s) {
+  if (rhs_mode) return launch_one<R, MIX, LES, VISC, true>(c, F, istage, alfa, beta, adt, kchunk, fl, false, slots, s);
+  return launch_one<R, MIX, LES, VISC, false>(c, F, istage, alfa, beta, adt, kchunk, fl, nv0, slots, s);
 }
 
-template struct StageLaunch<PartR, PART_MIX, PART_LES>;
+template struct StageLaunch<PartR, PART_MIX, PART_LES, PART_VISC>;
 
 #else  // CB_PART_BATCH
 
@@ -118,24 +113,21 @@ cudaError_t batched_attrs() {
 }
 }  // namespace
 
-template <typename R, bool MIX, bool LES>
-cudaError_t BatchLaunch<R, MIX, LES>::attrs() {
-  cudaError_t e = batched_attrs<R, MIX, LES, true>();
-  if (e == cudaSuccess) e = batched_attrs<R, MIX, LES, false>();
-  return e;
+template <typename R, bool MIX, bool LES, bool VISC>
+cudaError_t BatchLaunch<R, MIX, LES, VISC>::attrs() {
+  return batched_attrs<R, MIX, LES, VISC>();
 }
 
-template <typename R, bool MIX, bool LES>
-cudaError_t BatchLaunch<R, MIX, LES>::launch(const BatchBlock *tab, const int2 *items, int nitems, unsigned *counter,
-                                             int istage, double alfa, double beta, double adt, bool visc, int fl,
-                                             bool nv0, int ctas, cudaStream_t s) {
-  auto kern = visc ? batched_kernel<R, MIX, LES, true>(fl, nv0) : batched_kernel<R, MIX, LES, false>(fl, nv0);
-  kern<<<ctas, stage_threads<MIX>(fl), stage_smem_for<R, MIX>(fl, nv0), s>>>(tab, items, nitems, counter, istage, alfa, beta,
-                                                                       adt);
+template <typename R, bool MIX, bool LES, bool VISC>
+cudaError_t BatchLaunch<R, MIX, LES, VISC>::launch(const BatchBlock *tab, const int2 *items, int nitems, unsigned *counter,
+                                                   int istage, double alfa, double beta, double adt, int fl, bool nv0,
+                                                   int ctas, cudaStream_t s) {
+  batched_kernel<R, MIX, LES, VISC>(fl, nv0)<<<ctas, stage_threads<MIX>(fl), stage_smem_for<R, MIX>(fl, nv0), s>>>(
+      tab, items, nitems, counter, istage, alfa, beta, adt);
   return cudaGetLastError();
 }
 
-template struct BatchLaunch<PartR, PART_MIX, PART_LES>;
+template struct BatchLaunch<PartR, PART_MIX, PART_LES, PART_VISC>;
 
 #endif  // CB_PART_BATCH
 
