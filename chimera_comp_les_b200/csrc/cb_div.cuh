@@ -22,11 +22,21 @@
 // Rusanov 64^3 1.08 -> 0.63 ms; mixed form (the node reciprocal only) WENO5-JS
 // + Roe 192^3 7.97 -> 7.85 ms.
 //
-// Range: a zero, infinite, subnormal or NaN denominator (or a zero or
-// infinite radicand) gives NaN; callers for which that state can lead to a
-// finite result test the quotients with finite_hi and redo them by a / b.
+// Range: that holds for denominators and radicands with |b| in 2^-960 .. 2^960
+// (in_range) and finite numerators whose quotient does not overflow; below
+// |a| = 2^-960 the remainder may underflow and q miss its last bit.  For other
+// denominators the hardware approximations flush: a zero, infinite, subnormal or
+// NaN b gives NaN, one above 2^1022 the finite value 0.  So the stage kernels do
+// not rely on the result alone: every node's state is tested once, where it
+// enters the ring (wide_state), and what a face can cancel (densities, c^2) or
+// overflow is tested there; a tile march that met one out of bounds is done
+// again with a / b and sqrt (FLUX_IEEE).  The bounds on the nodes leave room for
+// everything the faces build from them: squared WENO smoothness measures stay
+// below 2^960, their weights and sums above 2^-960.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 namespace cb {
 
@@ -123,9 +133,29 @@ struct Den<double> {
   }
 };
 
+// The same by a / b: for values out of the branch-free quotients' range.  Out of
+// line, for code that hardly ever runs.
+template <typename R>
+static __device__ __noinline__ R plain_quot(R a, R b) { return a / b; }
+template <typename R>
+static __device__ __noinline__ R plain_root(R x) { return sqrt(x); }
+template <typename R>
+struct PlainDen {
+  R b;
+  __device__ __forceinline__ explicit PlainDen(R b_) : b(b_) {}
+  __device__ __forceinline__ PlainDen doubled() const { return PlainDen(R(2.0) * b); }
+  __device__ __forceinline__ R operator()(R a) const { return plain_quot(a, b); }
+};
+template <typename R, bool IEEE>
+using DenOf = std::conditional_t<IEEE, PlainDen<R>, Den<R>>;
+
 // a / 3 (FP64: with the reciprocal rounded to nearest)
-__device__ __forceinline__ double third(double a) { return Den<double>(3.0, 1.0 / 3.0)(a); }
-__device__ __forceinline__ float third(float a) { return a / 3.0f; }
+template <typename R, bool IEEE>
+__device__ __forceinline__ R third(R a) {
+  if constexpr (sizeof(R) == 4) return a / R(3.0);
+  else if constexpr (IEEE) return plain_quot(a, R(3.0));
+  else return Den<double>(3.0, 1.0 / 3.0)(a);
+}
 
 __device__ __forceinline__ double root(double x) {
   const double z = rsqrt_approx(x);
@@ -141,9 +171,33 @@ __device__ __forceinline__ float root(float x) {
   return g;
 }
 
+template <typename R, bool IEEE>
+__device__ __forceinline__ R root_of(R x) {
+  if constexpr (IEEE) return plain_root(x);
+  else return root(x);
+}
+
 // false for an infinity or a NaN
 __device__ __forceinline__ bool finite_hi(double x) {
   return ((unsigned)__double2hiint(x) & 0x7fffffffu) < 0x7ff00000u;
+}
+
+// the exponent bits of x above its sign-free high word: monotone in |x|
+__device__ __forceinline__ unsigned mag_hi(double x) { return (unsigned)__double2hiint(x) << 1; }
+__host__ __device__ constexpr unsigned mag_pow2(int e) { return (unsigned)(1023 + e) << 21; }  // mag_hi of 2^e
+// |b| in 2^-960 .. 2^960
+__device__ __forceinline__ bool in_range(double b) {
+  return mag_hi(b) - mag_pow2(-960) < mag_pow2(960) - mag_pow2(-960);
+}
+
+// Whether a node's conserved state v and pressure p lie outside |x| < 2^230,
+// |rho| >= 2^-500 (also true for a NaN).  Inside, rho's quotients are in range
+// and finite; differences of values square to at most 2^466 and, with the
+// smoothness measures' coefficients, (eps + beta)^2 stays below 2^932.
+__device__ __forceinline__ bool wide_state(const double *v, double p) {
+  const unsigned r = mag_hi(v[0]);
+  const unsigned a = max(max(r, mag_hi(v[1])), mag_hi(v[2])), b = max(max(mag_hi(v[3]), mag_hi(v[4])), mag_hi(p));
+  return max(a, b) >= mag_pow2(230) || r < mag_pow2(-500);
 }
 
 }  // namespace cb

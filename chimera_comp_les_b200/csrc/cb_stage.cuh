@@ -68,6 +68,10 @@ struct TileShape {
 // (fluxorder 3) -- the options the host checked, as compile-time constants, so
 // the kernel carries no other branch of them.
 constexpr int FLUX_ROE = 1, FLUX_SIGMA1 = 2, FLUX_SIGMA0 = 4, FLUX_W5 = 8, FLUX_PLAIN = 16, FLUX_W3 = 32;
+// FLUX_IEEE: every quotient and root by a / b and sqrt, for tiles with values out
+// of the branch-free ones' range (stage_kernel); FLUX_BLEND with it: the blend is
+// formed at every weight, as the right-hand side's kernels do
+constexpr int FLUX_IEEE = 64, FLUX_BLEND = 128;
 // the bits of a periodic or interface block's options (0: no PLAIN variant)
 inline int flux_plain_bits(int twod, int fluxorder, int weno_order) {
   if (twod != 0) return 0;
@@ -202,6 +206,7 @@ struct Ring {
   static constexpr int MPX = BX + 2, MPY = BY + 2, MPN = MPX * MPY;
   const float4 *mt;
   const double *nt;
+  int *wd;  // the march met a value out of the branch-free quotients' range
   __device__ __forceinline__ float4 met(int e, NRef n) const { return mt[e * MPN + (n.y - 1) * MPX + (n.x - 1)]; }
   __device__ __forceinline__ double nut(NRef n) const { return nt[(n.y - 1) * MPX + (n.x - 1)]; }
   // slot of relative plane r (-H .. NPL-H-1) is sb + r + H modulo NPL, with
@@ -273,22 +278,22 @@ template <typename R>
 __device__ __forceinline__ R muscl_l(R qm, R q0, R qp) { return q0 + R(0.5) * r_minmod(qp - q0, q0 - qm); }
 template <typename R>
 __device__ __forceinline__ R muscl_r(R qm, R q0, R qp) { return q0 - R(0.5) * r_minmod(qp - q0, q0 - qm); }
-template <typename R>
+template <typename R, class D = Den<R>>
 __device__ __forceinline__ R weno3_l(R qm, R q0, R qp) {
   const R d0 = R(0.6666667), d1 = R(0.3333333), eps = R(1e-6);  // rhs.c:2386 (truncated weights)
   R r0 = R(0.5) * q0 + R(0.5) * qp, r1 = R(-0.5) * qm + R(1.5) * q0;
   R b0 = (qp - q0) * (qp - q0), b1 = (qm - q0) * (qm - q0);
-  const R a0 = Den<R>((eps + b0) * (eps + b0))(d0), a1 = Den<R>((eps + b1) * (eps + b1))(d1);
-  const Den<R> as(a0 + a1);
+  const R a0 = D((eps + b0) * (eps + b0))(d0), a1 = D((eps + b1) * (eps + b1))(d1);
+  const D as(a0 + a1);
   return as(a0) * r0 + as(a1) * r1;
 }
-template <typename R>
+template <typename R, class D = Den<R>>
 __device__ __forceinline__ R weno3_r(R qm, R q0, R qp) {
   const R d0 = R(0.6666667), d1 = R(0.3333333), eps = R(1e-6);
   R r0 = R(1.5) * q0 - R(0.5) * qp, r1 = R(0.5) * qm + R(0.5) * q0;
   R b0 = (qp - q0) * (qp - q0), b1 = (qm - q0) * (qm - q0);
-  const R a0 = Den<R>((eps + b0) * (eps + b0))(d0), a1 = Den<R>((eps + b1) * (eps + b1))(d1);
-  const Den<R> as(a0 + a1);
+  const R a0 = D((eps + b0) * (eps + b0))(d0), a1 = D((eps + b1) * (eps + b1))(d1);
+  const D as(a0 + a1);
   return as(a0) * r0 + as(a1) * r1;
 }
 template <typename R>
@@ -309,7 +314,7 @@ __device__ __forceinline__ R eno_l(R qm, R q0, R qp, int k) {
 // eps = 1e-6, value sum(alpha_k q_k) / (6 sum(alpha_k)).  The right-biased
 // value at x_{i+1/2} is weno5(v_{i+3}, .., v_{i-1}).  Same operation order as
 // the oracle's restatement (bit-identical in the FP64 form).
-template <typename R>
+template <typename R, class D = Den<R>>
 __device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
   const R eps = R(1e-6), c13 = R(13.0 / 12.0);
   const R q0 = (R(2.0) * a - R(7.0) * b) + R(11.0) * c;
@@ -321,10 +326,10 @@ __device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
   const R b0 = c13 * (t0 * t0) + R(0.25) * (u0 * u0);
   const R b1 = c13 * (t1 * t1) + R(0.25) * (u1 * u1);
   const R b2 = c13 * (t2 * t2) + R(0.25) * (u2 * u2);
-  const R a0 = Den<R>((eps + b0) * (eps + b0))(R(0.1));
-  const R a1 = Den<R>((eps + b1) * (eps + b1))(R(0.6));
-  const R a2 = Den<R>((eps + b2) * (eps + b2))(R(0.3));
-  return Den<R>(R(6.0) * ((a0 + a1) + a2))((a0 * q0 + a1 * q1) + a2 * q2);
+  const R a0 = D((eps + b0) * (eps + b0))(R(0.1));
+  const R a1 = D((eps + b1) * (eps + b1))(R(0.6));
+  const R a2 = D((eps + b2) * (eps + b2))(R(0.3));
+  return D(R(6.0) * ((a0 + a1) + a2))((a0 * q0 + a1 * q1) + a2 * q2);
 }
 
 // The mixed form's MUSCL reconstruction of two fields at once:
@@ -388,11 +393,12 @@ __device__ __forceinline__ void weno3_2(float2 q0, float2 q1, float2 q2, float2 
 // reference state); pst/pin: the carried pressure of the FP64 form.  The
 // ring's derive pass and the global-memory path of far stencil nodes share
 // this arithmetic.
-template <typename R, bool MIX>
-__device__ __forceinline__ void node_qp(const DevCfg &c, const double v[5], bool pst, double pin, R q[5], R &p) {
+template <typename R, bool MIX, bool IEEE>
+__device__ __forceinline__ void node_qp(const DevCfg &c, const double v[5], bool pst, double pin, R q[5], R &p,
+                                        int *wd) {
   double pp = 0.0, e = v[4];
   if (v[0] != 0.0) {
-    const Den<double> rho(v[0]);
+    const DenOf<double, IEEE> rho(v[0]);
     if (MIX) {
       const double ri = rho(1.0);
       pp = (c.gamma - 1) * (v[4] - 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) * ri);
@@ -400,9 +406,8 @@ __device__ __forceinline__ void node_qp(const DevCfg &c, const double v[5], bool
       pp -= c.p_ref;
     } else {
       const double ke = 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
-      double kr = rho(ke);
-      if (!finite_hi(kr)) kr = ke / v[0];
-      pp = pst ? pin : (c.gamma - 1) * (v[4] - kr);
+      pp = pst ? pin : (c.gamma - 1) * (v[4] - rho(ke));
+      if (!IEEE && wide_state(v, pp)) *wd = 1;
     }
   }
 #pragma unroll
@@ -417,17 +422,9 @@ __device__ __forceinline__ void node_qp(const DevCfg &c, const double v[5], bool
 // face velocity measure 0.5*(uconL + uconR) that multiplies H_ref.
 // The mixed form multiplies by one reciprocal of each state's density
 // instead of dividing by it four times (FP32 rounding differences only).
-// One side's face velocity and sound speed sqrt(|gamma p / rho| h.h) by a / b
-// and sqrt: where the branch-free quotients and roots leave their range (zero
-// or non-finite density or sound speed).
-static __device__ __noinline__ double2 side_speed_ieee(double r, double ru, double rv, double rw, double p, double h0,
-                                                       double h1, double h2) {
-  const double u = h0 * (ru / r) + h1 * (rv / r) + h2 * (rw / r);
-  const double cc = GAMMA_CONV * p / r, gii = h0 * h0 + h1 * h1 + h2 * h2;
-  return make_double2(u, sqrt(fabs(cc) * gii));
-}
-template <typename R, bool MIX>
-__device__ __forceinline__ void rusanov(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
+// Returns whether the quotients and roots were in range (FP64 form).
+template <typename R, bool MIX, bool IEEE>
+__device__ __forceinline__ bool rusanov(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
                                         bool r_from_l, R pref, R F[5], R &Uf) {
   R uconL, uconR, saL, saR;
   const R gii = h[0] * h[0] + h[1] * h[1] + h[2] * h[2];
@@ -441,20 +438,12 @@ __device__ __forceinline__ void rusanov(const R QL[5], const R QR[5], R pL, R pR
     saL = fabs(uconL) + root(fabs(cL) * gii);
     saR = fabs(uconR) + root(fabs(cR) * gii);
   } else {
-    const Den<R> rl(QL[0]), rr(QR[0]);
+    const DenOf<R, IEEE> rl(QL[0]), rr(QR[0]);
     const R UR = h[0] * rr(QR[1]) + h[1] * rr(QR[2]) + h[2] * rr(QR[3]);
     uconL = use_qr_for_l ? UR : h[0] * rl(QL[1]) + h[1] * rl(QL[2]) + h[2] * rl(QL[3]);
     uconR = r_from_l ? uconL : UR;
-    saL = fabs(uconL) + root(fabs(rl(R(GAMMA_CONV) * pL)) * gii);
-    saR = fabs(uconR) + root(fabs(rr(R(GAMMA_CONV) * pR)) * gii);
-    if (!(finite_hi(saL) && finite_hi(saR))) {
-      const double2 l = side_speed_ieee(QL[0], QL[1], QL[2], QL[3], pL, h[0], h[1], h[2]);
-      const double2 r = side_speed_ieee(QR[0], QR[1], QR[2], QR[3], pR, h[0], h[1], h[2]);
-      uconL = use_qr_for_l ? r.x : l.x;
-      uconR = r_from_l ? uconL : r.x;
-      saL = fabs(uconL) + l.y;
-      saR = fabs(uconR) + r.y;
-    }
+    saL = fabs(uconL) + root_of<R, IEEE>(fabs(rl(R(GAMMA_CONV) * pL)) * gii);
+    saR = fabs(uconR) + root_of<R, IEEE>(fabs(rr(R(GAMMA_CONV) * pR)) * gii);
   }
   R SA = (saL < saR) ? saR : saL;
   F[0] = R(0.5) * (QL[0] * uconL + QR[0] * uconR) - R(0.5) * SA * (QR[0] - QL[0]);
@@ -463,6 +452,7 @@ __device__ __forceinline__ void rusanov(const R QL[5], const R QR[5], R pL, R pR
     F[1 + a] = R(0.5) * ((QL[1 + a] * uconL + QR[1 + a] * uconR) + (pL * h[a] + pR * h[a])) - R(0.5) * SA * (QR[1 + a] - QL[1 + a]);
   F[4] = R(0.5) * ((pL + QL[4]) * uconL + (pR + QR[4]) * uconR) - R(0.5) * SA * (QR[4] - QL[4]);
   Uf = MIX ? R(0.5) * (uconL + uconR) : R(0);
+  return MIX || (finite_hi(saL) && finite_hi(saR));
 }
 
 // Roe's approximate Riemann solver with Harten's entropy fix (no counterpart
@@ -472,24 +462,13 @@ __device__ __forceinline__ void rusanov(const R QL[5], const R QR[5], R pL, R pR
 // Roe-averaged Jacobian along n = h/|h|, acoustic speeds below 0.1 c~
 // smoothed to (l^2 + delta^2) / (2 delta).  Mixed form: the enthalpy adds
 // back H_ref; pressure and energy differences are shift-free.
-// The FP64 form's quotients and roots are the branch-free ones (cb_div.cuh);
-// IEEE: a / b and sqrt, for the states where those leave their range.
-template <typename R>
-struct PlainDen {
-  R b;
-  __device__ __forceinline__ explicit PlainDen(R b_) : b(b_) {}
-  __device__ __forceinline__ PlainDen doubled() const { return PlainDen(R(2.0) * b); }
-  __device__ __forceinline__ R operator()(R a) const { return a / b; }
-};
+// Returns whether the quotients and roots were in range (FP64 form).
 template <typename R, bool MIX, bool IEEE>
-__device__ __forceinline__ void roe_flux(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
-                                         bool r_from_l, R href, R F[5], R &Uf) {
+__device__ __forceinline__ bool roe(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
+                                    bool r_from_l, R href, R F[5], R &Uf) {
   const R g = R(GAMMA_CONV);
-  using D = std::conditional_t<IEEE, PlainDen<R>, Den<R>>;
-  auto rt_of = [](R x) -> R {
-    if constexpr (IEEE) return sqrt(x);
-    else return root(x);
-  };
+  using D = DenOf<R, IEEE>;
+  auto rt_of = [](R x) -> R { return root_of<R, IEEE>(x); };
   const D dl(QL[0]), dr_(QR[0]);
   // the mixed form multiplies by reciprocals of the densities, the face area
   // and the root sum (FP32 rounding differences only)
@@ -539,38 +518,7 @@ __device__ __forceinline__ void roe_flux(const R QL[5], const R QR[5], R pL, R p
     F[1 + a] = R(0.5) * ((QL[1 + a] * uconL + QR[1 + a] * uconR) + (pL * h[a] + pR * h[a])) - R(0.5) * area * D5[1 + a];
   F[4] = R(0.5) * ((pL + QL[4]) * uconL + (pR + QR[4]) * uconR) - R(0.5) * area * D5[4];
   Uf = MIX ? R(0.5) * (uconL + uconR) : R(0);
-}
-struct RoeIn {
-  double QL[5], QR[5], pL, pR, h[3];
-  bool use_qr_for_l, r_from_l;
-};
-struct RoeOut {
-  double F[5];
-};
-static __device__ __noinline__ RoeOut roe_ieee(const RoeIn in) {
-  RoeOut o;
-  double uf;
-  roe_flux<double, false, true>(in.QL, in.QR, in.pL, in.pR, in.h, in.use_qr_for_l, in.r_from_l, 0.0, o.F, uf);
-  return o;
-}
-template <typename R, bool MIX>
-__device__ __forceinline__ void roe(const R QL[5], const R QR[5], R pL, R pR, const R h[3], bool use_qr_for_l,
-                                    bool r_from_l, R href, R F[5], R &Uf) {
-  roe_flux<R, MIX, false>(QL, QR, pL, pR, h, use_qr_for_l, r_from_l, href, F, Uf);
-  if constexpr (!MIX) {
-    if (!(finite_hi(F[0]) && finite_hi(F[1]) && finite_hi(F[2]) && finite_hi(F[3]) && finite_hi(F[4]))) {
-      RoeIn in;
-#pragma unroll
-      for (int q = 0; q < 5; q++) { in.QL[q] = QL[q]; in.QR[q] = QR[q]; }
-#pragma unroll
-      for (int q = 0; q < 3; q++) in.h[q] = h[q];
-      in.pL = pL; in.pR = pR;
-      in.use_qr_for_l = use_qr_for_l; in.r_from_l = r_from_l;
-      const RoeOut o = roe_ieee(in);
-#pragma unroll
-      for (int q = 0; q < 5; q++) F[q] = o.F[q];
-    }
-  }
+  return MIX || (in_range(c2) && finite_hi(F[0]) && finite_hi(F[1]) && finite_hi(F[2]) && finite_hi(F[3]) && finite_hi(F[4]));
 }
 
 // ------------------------------------------------------- inviscid face ----
@@ -580,7 +528,7 @@ __device__ __forceinline__ void roe(const R QL[5], const R QR[5], R pL, R pR, co
 // a wall node (nvert > 2.9).  Offsets -2 and +3 come from the ring when it
 // holds them (always along k) and otherwise from global memory through the
 // ring's own node arithmetic.
-template <typename R, bool MIX, bool NV0, class RG>
+template <typename R, bool MIX, bool NV0, bool IEEE, class RG>
 __device__ __forceinline__ bool weno5_face(const DevCfg &c, const DevFields &F, const RG &Rg, NRef a, int d, int pos,
                                            int m, long long g0, long long sd, const R Q[4][5], const R P[4], R QL[5],
                                            R QR[5], R &pL, R &pR) {
@@ -608,9 +556,10 @@ __device__ __forceinline__ bool weno5_face(const DevCfg &c, const DevFields &F, 
       double v[5];
 #pragma unroll
       for (int q = 0; q < 5; q++) v[q] = ldg(F.q[q] + g);
-      node_qp<R, MIX>(c, v, pst, pst ? ldg(F.pin + g) : 0.0, qd, pd);
+      node_qp<R, MIX, IEEE>(c, v, pst, pst ? ldg(F.pin + g) : 0.0, qd, pd, Rg.wd);
     }
   }
+  using D = DenOf<R, IEEE>;
   if constexpr (MIX) {  // fields two at a time; the pressure is the energy's partner
 #pragma unroll
     for (int q = 0; q < 6; q += 2) {
@@ -625,11 +574,11 @@ __device__ __forceinline__ bool weno5_face(const DevCfg &c, const DevFields &F, 
   } else {
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-      QL[q] = weno5(Qm[q], Q[0][q], Q[1][q], Q[2][q], Q[3][q]);
-      QR[q] = weno5(Qp[q], Q[3][q], Q[2][q], Q[1][q], Q[0][q]);
+      QL[q] = weno5<R, D>(Qm[q], Q[0][q], Q[1][q], Q[2][q], Q[3][q]);
+      QR[q] = weno5<R, D>(Qp[q], Q[3][q], Q[2][q], Q[1][q], Q[0][q]);
     }
-    pL = weno5(Pm, P[0], P[1], P[2], P[3]);
-    pR = weno5(Pp, P[3], P[2], P[1], P[0]);
+    pL = weno5<R, D>(Pm, P[0], P[1], P[2], P[3]);
+    pR = weno5<R, D>(Pp, P[3], P[2], P[1], P[0]);
   }
   return true;
 }
@@ -648,6 +597,14 @@ __device__ __forceinline__ bool weno5_face(const DevCfg &c, const DevFields &F, 
 // faces whose six-node stencil pos-2 .. pos+3 lies on the nodes 0 .. m-1 and
 // holds no wall node take WENO5-JS; the others keep the reference's path, and
 // the (j < 30 && k < 7) MUSCL override of the non-LES scheme is off.
+// the blend weight when it is one constant on every face (as the host chooses
+// FLUX_SIGMA1 / FLUX_SIGMA0), else -1
+__device__ __forceinline__ double constant_weight(const DevCfg &c) {
+  return !c.calc_sigma && c.s_x == c.s_y && c.s_y == c.s_z ? c.s_x : -1.;
+}
+// *w = 1.  Out of line: with a plain store the variants with boundary codes and
+// both fluxes spill 100 B more (channel 64x65x96 0.643 -> 0.665 ms per step).
+static __device__ __noinline__ void mark(int *w) { *w = 1; }
 template <typename R, bool MIX, bool LES, class RG, int DIR, int FLUX = 0, bool NV0 = false>
 __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, const RG &Rg, NRef a,
                                           int gi, int gj, int gk, int drt, R Fc[5]) {
@@ -693,6 +650,8 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
   constexpr bool W5 = (FLUX & FLUX_W5) != 0;
   constexpr bool CEN_ONLY = LES && (FLUX & FLUX_SIGMA1) != 0;
   constexpr bool UPW_ONLY = LES && (FLUX & FLUX_SIGMA0) != 0;
+  constexpr bool IEEE = (FLUX & FLUX_IEEE) != 0;
+  using D = DenOf<R, IEEE>;
   R Fw[5], Ufw = R(0);
 #pragma unroll
   for (int q = 0; q < 5; q++) Fw[q] = R(0);
@@ -747,7 +706,7 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
         pL = muscl_l(wm ? P[2] : P[0], P[1], P[2]);
         pR = muscl_r(P[1], P[2], wp ? P[1] : P[3]);
       }
-    } else if (W5 && weno5_face<R, MIX, NV0>(c, F, Rg, a, d, pos, m, g0, sd, Q, P, QL, QR, pL, pR)) {
+    } else if (W5 && weno5_face<R, MIX, NV0, IEEE>(c, F, Rg, a, d, pos, m, g0, sd, Q, P, QL, QR, pL, pR)) {
       // WENO5-JS reconstruction of Q and p
     } else if (MIX && NV0) {
       if constexpr (MIX) {  // WENO3 without walls, fields two at a time
@@ -778,8 +737,8 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
         pL = eno_l(P[1], P[2], P[3], ord);
       } else {
   #pragma unroll
-        for (int q = 0; q < 5; q++) QL[q] = weno3_l(Q[0][q], Q[1][q], Q[2][q]);
-        pL = weno3_l(P[0], P[1], P[2]);
+        for (int q = 0; q < 5; q++) QL[q] = weno3_l<R, D>(Q[0][q], Q[1][q], Q[2][q]);
+        pL = weno3_l<R, D>(P[0], P[1], P[2]);
         if (!LES && !PLAIN && d == 1 && gj == 1 && c.isothermal && c.bctype[2] == 1) {  // rhs.c:2926
           QL[0] = eno_l(Q[1][0], Q[2][0], Q[3][0], ord);
           QL[4] = eno_l(Q[1][4], Q[2][4], Q[3][4], ord);
@@ -792,19 +751,21 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
         pR = eno_r(P[0], P[1], P[2], ord);
       } else {
   #pragma unroll
-        for (int q = 0; q < 5; q++) QR[q] = weno3_r(Q[1][q], Q[2][q], Q[3][q]);
-        pR = weno3_r(P[1], P[2], P[3]);
+        for (int q = 0; q < 5; q++) QR[q] = weno3_r<R, D>(Q[1][q], Q[2][q], Q[3][q]);
+        pR = weno3_r<R, D>(P[1], P[2], P[3]);
       }
     }
+    bool ok;
     if (LES) {
-      if (ROE) roe<R, MIX>(QL, QR, pL, pR, h, false, false, href, Fw, Ufw);
-      else rusanov<R, MIX>(QL, QR, pL, pR, h, false, false, pref, Fw, Ufw);
+      if (ROE) ok = roe<R, MIX, IEEE>(QL, QR, pL, pR, h, false, false, href, Fw, Ufw);
+      else ok = rusanov<R, MIX, IEEE>(QL, QR, pL, pR, h, false, false, pref, Fw, Ufw);
     } else {
       const bool use_qr_l = !PLAIN && (pos == m - 2 && bc_hi(c, d) == 1);
       const bool r_from_l = !PLAIN && (pos == 0 && bc_lo(c, d) == 1);
-      if (ROE) roe<R, MIX>(QL, QR, pL, pR, h, use_qr_l, r_from_l, href, Fw, Ufw);
-      else rusanov<R, MIX>(QL, QR, pL, pR, h, use_qr_l, r_from_l, pref, Fw, Ufw);
+      if (ROE) ok = roe<R, MIX, IEEE>(QL, QR, pL, pR, h, use_qr_l, r_from_l, href, Fw, Ufw);
+      else ok = rusanov<R, MIX, IEEE>(QL, QR, pL, pR, h, use_qr_l, r_from_l, pref, Fw, Ufw);
     }
+    if (!IEEE && !ok && (nv0 < BLANK || nv1 < BLANK)) mark(Rg.wd);
   }
   if (!LES) {
 #pragma unroll
@@ -813,7 +774,9 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
     return;
   }
 
-  if constexpr (UPW_ONLY) {
+  // (FLUX_IEEE has one variant for all blend weights)
+  const double sw = IEEE && (FLUX & FLUX_BLEND) == 0 ? constant_weight(c) : -1.;
+  if (UPW_ONLY || sw == 0.) {
 #pragma unroll
     for (int q = 0; q < 5; q++) Fc[q] = Fw[q];
     if (MIX) Fc[4] += href * Ufw;
@@ -853,12 +816,12 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
 #pragma unroll
     for (int s = 0; s < 4; s++) {
       const MetV<R> ms = s == 1 ? m0 : (s == 2 ? m1 : met_load<R, MIX>(F, d, g0 + (s - 1) * sd));
-      U[s] = Den<R>(Q[s][0])(R(1.)) * (ms.x * Q[s][1] + ms.y * Q[s][2] + ms.z * Q[s][3]);
+      U[s] = D(Q[s][0])(R(1.)) * (ms.x * Q[s][1] + ms.y * Q[s][2] + ms.z * Q[s][3]);
       EP[s] = P[s] + Q[s][4];
     }
     const R fp4 = R(1.0) / R(12.0) * (-P[0] + R(7) * P[1] + R(7) * P[2] - P[3]);
     if (c.central == 2) {
-#define CB_FP2(A0, A1, A2, A3) (third((A1 + A2) * (U[1] + U[2])) - R(1.) / R(24.) * (A0 * U[0] + A0 * U[2] + A1 * U[1] + A1 * U[3] + A2 * U[2] + A2 * U[0] + A3 * U[1] + A3 * U[3]))
+#define CB_FP2(A0, A1, A2, A3) (third<R, IEEE>((A1 + A2) * (U[1] + U[2])) - R(1.) / R(24.) * (A0 * U[0] + A0 * U[2] + A1 * U[1] + A1 * U[3] + A2 * U[2] + A2 * U[0] + A3 * U[1] + A3 * U[3]))
       Fcen[0] = CB_FP2(Q[0][0], Q[1][0], Q[2][0], Q[3][0]);
       Fcen[1] = CB_FP2(Q[0][1], Q[1][1], Q[2][1], Q[3][1]) + fp4 * h[0];
       Fcen[2] = CB_FP2(Q[0][2], Q[1][2], Q[2][2], Q[3][2]) + fp4 * h[1];
@@ -879,7 +842,7 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
   } else {
     const R rc = R(0.5) * (Q[1][0] + Q[2][0]), uc = R(0.5) * (Q[1][1] + Q[2][1]), vc = R(0.5) * (Q[1][2] + Q[2][2]);
     const R wc = R(0.5) * (Q[1][3] + Q[2][3]), ec = R(0.5) * (Q[1][4] + Q[2][4]);
-    const R Uc = Den<R>(rc)(h[0] * uc + h[1] * vc + h[2] * wc);
+    const R Uc = D(rc)(h[0] * uc + h[1] * vc + h[2] * wc);
     const R pa = R(0.5) * (P[1] + P[2]);
     Fcen[0] = rc * Uc;
     Fcen[1] = uc * Uc + pa * h[0];
@@ -888,7 +851,7 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
     Fcen[4] = Uc * (ec + pa);
     Ufc = MIX ? Uc : R(0);
   }
-  if constexpr (CEN_ONLY) {
+  if (CEN_ONLY || sw == 1.) {
 #pragma unroll
     for (int q = 0; q < 5; q++) Fc[q] = Fcen[q];
     if (MIX) Fc[4] += href * Ufc;
@@ -913,6 +876,7 @@ template <typename R, bool MIX, bool LES, class RG, int DIR, bool NV0 = false, i
 __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, const RG &Rg, NRef a,
                                           int gi, int gj, int gk, int drt, R Fv[5], R A[3]) {
   constexpr bool SMET = StageMet<MIX, NV0, FLUX>::on;
+  constexpr bool IEEE = (FLUX & FLUX_IEEE) != 0;
   static_assert(!SMET || (MIX && DIR >= 0), "the metric slot holds FP32 vectors, selected at compile time");
   const int d = DIR >= 0 ? DIR : drt;
   const long long g0 = gidx(c, gi, gj, gk), sd = gstride(c, d), g1 = g0 + sd;
@@ -1087,8 +1051,12 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
   if constexpr (MIX) {
     heat = nu * R(c.kheat);
   } else {  // gamma * nu / Pr / (gamma - 1)
-    heat = Den<double>(c.gm1, c.r_gm1)(Den<double>(c.pr, c.r_pr)(c.gamma * nu));
-    if (!finite_hi(heat)) heat = c.gamma * nu / c.pr / c.gm1;
+    if constexpr (IEEE) {
+      heat = plain_quot(plain_quot(c.gamma * nu, c.pr), c.gm1);
+    } else {
+      heat = Den<double>(c.gm1, c.r_gm1)(Den<double>(c.pr, c.r_pr)(c.gamma * nu));
+      if (!finite_hi(heat)) *Rg.wd = 1;
+    }
   }
   Fv[4] = (Fv[1] * uh[0] + Fv[2] * uh[1] + Fv[3] * uh[2]) +
           (g11 * dpdc + g21 * dpde + g31 * dpdz) * ajc * heat;
@@ -1118,7 +1086,7 @@ __device__ __forceinline__ void visc_face(const DevCfg &c, const DevFields &F, c
       const R tx = (tu - div * md0) * ajc * (nut * rho_c);
       const R ty = (tv - div * md1) * ajc * (nut * rho_c);
       const R tz = (tw - div * md2) * ajc * (nut * rho_c);
-      const R sgs = third(-S2 * pf * R(c.ci) * R(2.0));
+      const R sgs = third<R, IEEE>(-S2 * pf * R(c.ci) * R(2.0));
       A[0] = tx + sgs * md0 * rho_c * sigma_c;
       A[1] = ty + sgs * md1 * rho_c * sigma_c;
       A[2] = tz + sgs * md2 * rho_c * sigma_c;
@@ -1305,8 +1273,9 @@ __device__ __forceinline__ void plane_faces(const DevCfg &c, const DevFields &F,
         // one instantiation per direction (d is warp-uniform): the index
         // arithmetic of every stencil shift folds into constants (4 % faster
         // than one copy for all directions at 128 registers); the WENO5-JS
-        // variants, at 168 registers, keep one copy (13 % faster there)
-        if constexpr ((FLUX & FLUX_W5) != 0)
+        // variants, at 168 registers, keep one copy (13 % faster there), and so
+        // does the code that hardly ever runs
+        if constexpr ((FLUX & (FLUX_W5 | FLUX_IEEE)) != 0)
           face_flux_half<R, MIX, LES, VISC, RG, -1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, conv, Gf);
         else if (d == 0) face_flux_half<R, MIX, LES, VISC, RG, 0, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, conv, Gf);
         else if (d == 1) face_flux_half<R, MIX, LES, VISC, RG, 1, FLUX, NV0>(c, F, Rg, a, fi, fj, k, d, conv, Gf);
@@ -1353,10 +1322,14 @@ __device__ __forceinline__ void plane_faces(const DevCfg &c, const DevFields &F,
 
 
 // One tile column (bxi, byi) of one block over the planes kb .. ke-1: the
-// whole k march, with its prologue.
+// whole k march, with its prologue and a barrier at its end.  *again: set when the
+// results do not stand (stage_kernel).
 template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX = 0, bool NV0 = false>
 __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, int bxi, int byi, int kb, int ke,
-                                           int istage, double alfa, double beta, double adt, double *smem_d) {
+                                           int istage, double alfa, double beta, double adt, double *smem_d,
+                                           int *again) {
+  constexpr bool IEEE = (FLUX & FLUX_IEEE) != 0;
+  constexpr bool CHECKED = !IEEE && !MIX;
   using G = StageGeo<FLUX>;
   constexpr int BX = G::BX, BY = G::BY, NPL = G::NPL, H = G::H;
   constexpr int NT = StageThreads<FLUX, MIX>::N;  // threads of the block
@@ -1377,6 +1350,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
   Rg.pl = smem;
   Rg.mt = mts;
   Rg.nt = nts;
+  Rg.wd = again;
   R *gxb = smem + (size_t)NPL * NF * PN;  // [NG][NXF]
   R *gyb = gxb + (size_t)NG * NXF;        // [NG][NYF]
   R *gzb = gyb + (size_t)NG * NYF;        // [NG][NZF] (not with the metric slot)
@@ -1433,27 +1407,21 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
           // one FP64 reciprocal instead of five divisions: the products differ
           // from the quotients by at most an FP64 ulp, far below the FP32
           // rounding of the shifted values stored next
-          const double ri = Den<double>(r)(1.0);
+          const double ri = DenOf<double, IEEE>(r)(1.0);
           v[F_P] = (c.gamma - 1) * (v[4] - 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]) * ri);
           v[F_U] = v[1] * ri;
           v[F_V] = v[2] * ri;
           v[F_W] = v[3] * ri;
           v[F_T] = v[F_P] * ri;
         } else {  // the reference's quotients (EqOfState rhs.c:4850, CalcUCat rhs.c:1349)
-          const Den<double> rho(r);
+          const DenOf<double, IEEE> rho(r);
           const double ke = 0.5 * (v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
           v[F_P] = pst ? pn : (c.gamma - 1) * (v[4] - rho(ke));
           v[F_U] = rho(v[1]);
           v[F_V] = rho(v[2]);
           v[F_W] = rho(v[3]);
           v[F_T] = rho(v[F_P]);
-          if (!(finite_hi(v[F_U]) && finite_hi(v[F_V]) && finite_hi(v[F_W]) && finite_hi(v[F_T]))) {
-            v[F_P] = pst ? pn : (c.gamma - 1) * (v[4] - ke / r);
-            v[F_U] = v[1] / r;
-            v[F_V] = v[2] / r;
-            v[F_W] = v[3] / r;
-            v[F_T] = v[F_P] / r;
-          }
+          if (!IEEE && wide_state(v, v[F_P])) *Rg.wd = 1;
         }
         if (MIX) {
           v[F_RE] -= c.e_ref;
@@ -1730,7 +1698,10 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
         if (!isfinite(out[0] + out[1] + out[2] + out[3] + out[4])) st |= ST_NONFINITE;
         if (!(out[0] > 0.)) st |= ST_NEG_RHO;
         if (!(p > 0.)) st |= ST_NEG_P;
-        if (st) atomicOr(F.status, st);
+        if (st != 0) {
+          if constexpr (CHECKED) *again = 1;
+          else atomicOr(F.status, st);
+        }
       }
 #pragma unroll
       for (int q = 0; q < NG; q++) Gzp[q] = SMET ? gzr[q] : gzb[(size_t)q * NZF + fz];
@@ -1756,11 +1727,9 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
 // planes beside dirty ones stays with them: a piece of its own costs a
 // prologue, about one plane.
 constexpr int MASK_MIN_RUN = 5;
-template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX = 0, bool NV0 = false>
-static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThreads<FLUX, MIX>::MIN_BLOCKS)
-    stage_kernel(const DevCfg c, const DevFields F, int istage, double alfa, double beta, double adt, int kchunk) {
-  extern __shared__ double smem_d[];
-  pdl_wait();
+template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX, bool NV0>
+__device__ __forceinline__ void stage_block(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta,
+                                            double adt, int kchunk, double *smem_d, int *again) {
   constexpr int BY = StageGeo<FLUX>::BY;
   const int nk = c.mz - 2, tiles_x = (c.mx - 2 + SBX - 1) / SBX;
   long long s, e;  // range of (column, plane) units, column-major
@@ -1779,7 +1748,7 @@ static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThread
     const int col = (int)(s / nk), k0 = (int)(s - (long long)col * nk);
     int k1 = (int)min((long long)nk, k0 + (e - s));
     bool clean = NV0;
-    if constexpr (!NV0) {
+    if constexpr (!NV0 && (FLUX & FLUX_IEEE) == 0) {
       int lo = 0, hi = nk;  // dirty planes lo .. hi - 1 of the column
       if (F.mask_planes != nullptr) { const int2 d = F.mask_planes[col]; lo = d.x; hi = d.y; }
       else if (F.all_clean) hi = 0;
@@ -1789,14 +1758,50 @@ static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThread
       else if (lo - k0 >= MASK_MIN_RUN) { clean = true; k1 = lo; }
       else if (k1 - hi >= MASK_MIN_RUN) k1 = hi;
     }
-    if (clean)
-      stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, true>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage,
-                                                          alfa, beta, adt, smem_d);
-    else if constexpr (!NV0)
-      stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, false>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage,
-                                                           alfa, beta, adt, smem_d);
+    if constexpr (NV0 || (FLUX & FLUX_IEEE) == 0)
+      if (clean)
+        stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, true>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage,
+                                                            alfa, beta, adt, smem_d, again);
+    if constexpr (!NV0)
+      if (!clean)
+        stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, false>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage,
+                                                             alfa, beta, adt, smem_d, again);
     s += k1 - k0;
   }
+}
+
+// A CTA's tiles again by a / b and sqrt, out of line: one variant for the PLAIN,
+// WENO3 and constant-weight ones (its blend skips what those skip; FLUX_BLEND:
+// the kernels without constant-weight variants).
+template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX, bool NV0>
+static __device__ __noinline__ void stage_again(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta,
+                                                double adt, int kchunk) {
+  extern __shared__ double smem_d[];
+  stage_block<R, MIX, LES, VISC, RHS_MODE, FLUX, NV0>(c, F, istage, alfa, beta, adt, kchunk, smem_d, nullptr);
+}
+__host__ __device__ constexpr int ieee_flux(int fl, bool blend) { return FLUX_IEEE | (blend ? FLUX_BLEND : 0) | (fl & (FLUX_ROE | FLUX_W5)); }
+
+// A CTA whose marches met values out of the range of the branch-free quotients,
+// or formed a state that the status word reports, does its tiles again with IEEE
+// quotients: they read Q and Qold and write qout or rhs only, so the first
+// results are overwritten.  The call stands at the kernel's end, where no value
+// lives across it (inside the loop over the tiles: MUSCL 128^3 3 % slower,
+// WENO5-JS + Roe 96^3 10 %).
+template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX = 0, bool NV0 = false>
+static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThreads<FLUX, MIX>::MIN_BLOCKS)
+    stage_kernel(const __grid_constant__ DevCfg c, const __grid_constant__ DevFields F, int istage, double alfa, double beta,
+                 double adt, int kchunk) {
+  extern __shared__ double smem_d[];
+  __shared__ int again;
+  if constexpr (!MIX) {
+    if (threadIdx.x == 0) again = 0;
+    __syncthreads();
+  }
+  pdl_wait();
+  stage_block<R, MIX, LES, VISC, RHS_MODE, FLUX, NV0>(c, F, istage, alfa, beta, adt, kchunk, smem_d, &again);
+  if constexpr (!MIX)
+    if (again)  // (every march ends with a barrier)
+      stage_again<R, MIX, LES, VISC, RHS_MODE, ieee_flux(FLUX, RHS_MODE), NV0>(c, F, istage, alfa, beta, adt, kchunk);
 }
 
 // The dirty planes of each tile column (a block per column): plane k (0-based
@@ -1921,6 +1926,33 @@ struct BatchBlock {
   long long first_item;  // index of this block's first item in the global list
 };
 
+// the march of one item; bb: the block's entry in shared memory
+template <typename R, bool MIX, bool LES, bool VISC, int FLUX, bool NV0>
+__device__ __forceinline__ void batch_item(const BatchBlock *blocks, int2 ib, BatchBlock &bb, int istage, double alfa,
+                                           double beta, double adt, double *smem_d, int *again) {
+  if (threadIdx.x == 0) bb = blocks[ib.x];
+  __syncthreads();
+  const int txy = bb.tiles_x * bb.tiles_y;
+  const int bzi = ib.y / txy, rem = ib.y - bzi * txy;
+  const int byi = rem / bb.tiles_x, bxi = rem - byi * bb.tiles_x;
+  const int kb = 1 + bzi * bb.kchunk;
+  stage_tile<R, MIX, LES, VISC, false, FLUX, NV0>(bb.c, bb.F, bxi, byi, kb, min(bb.c.mz - 1, kb + bb.kchunk), istage, alfa,
+                                                 beta, adt, smem_d, again);
+}
+
+// Items whose results do not stand (stage_kernel) are listed, and done again when
+// the list is full or the items are exhausted.
+struct BatchList {
+  int again, n, it[62];
+};
+template <typename R, bool MIX, bool LES, bool VISC, int FLUX, bool NV0>
+static __device__ __noinline__ void batch_again(const BatchBlock *blocks, const int2 *items, const BatchList &list,
+                                                BatchBlock &bb, int istage, double alfa, double beta, double adt) {
+  extern __shared__ double smem_d[];
+  for (int x = 0; x < list.n; x++)
+    batch_item<R, MIX, LES, VISC, FLUX, NV0>(blocks, items[list.it[x]], bb, istage, alfa, beta, adt, smem_d, nullptr);
+}
+
 template <typename R, bool MIX, bool LES, bool VISC, bool NV0 = false, int FLUX = 0>
 static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThreads<FLUX, MIX>::MIN_BLOCKS)
     stage_batched_kernel(const BatchBlock *__restrict__ blocks, const int2 *__restrict__ items, int nitems,
@@ -1928,21 +1960,30 @@ static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThread
   extern __shared__ double smem_d[];
   __shared__ BatchBlock bb;
   __shared__ int item;
-  for (;;) {
-    if (threadIdx.x == 0) item = (int)atomicAdd(counter, 1u);
-    __syncthreads();
-    const int it = item;
-    if (it >= nitems) break;
-    const int2 ib = items[it];  // (block, local item index)
-    if (threadIdx.x == 0) bb = blocks[ib.x];
-    __syncthreads();
-    const int txy = bb.tiles_x * bb.tiles_y;
-    const int bzi = ib.y / txy, rem = ib.y - bzi * txy;
-    const int byi = rem / bb.tiles_x, bxi = rem - byi * bb.tiles_x;
-    const int kb = 1 + bzi * bb.kchunk;
-    stage_tile<R, MIX, LES, VISC, false, FLUX, NV0>(bb.c, bb.F, bxi, byi, kb, min(bb.c.mz - 1, kb + bb.kchunk), istage,
-                                                   alfa, beta, adt, smem_d);
-    __syncthreads();  // bb and item are rewritten by the next iteration
+  __shared__ BatchList list;
+  for (bool more = true; more;) {
+    if (threadIdx.x == 0) list.n = 0;
+    for (;;) {
+      if (threadIdx.x == 0) {
+        item = (int)atomicAdd(counter, 1u);
+        list.again = 0;
+      }
+      __syncthreads();
+      const int it = item;
+      if (it >= nitems) {
+        more = false;
+        break;
+      }
+      batch_item<R, MIX, LES, VISC, FLUX, NV0>(blocks, items[it], bb, istage, alfa, beta, adt, smem_d, &list.again);
+      if (!MIX && threadIdx.x == 0 && list.again) list.it[list.n++] = it;
+      __syncthreads();  // bb and item are rewritten by the next iteration
+      if (!MIX && list.n == 62) break;
+    }
+    if constexpr (!MIX) {
+      if (list.n > 0)
+        batch_again<R, MIX, LES, VISC, ieee_flux(FLUX, !NV0), NV0>(blocks, items, list, bb, istage, alfa, beta, adt);
+      __syncthreads();
+    }
   }
 }
 
