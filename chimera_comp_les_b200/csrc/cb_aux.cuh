@@ -575,14 +575,19 @@ static __global__ void ghost_fill_kernel(const DevCfg c, double *const *planes, 
 // metrics, aj, filter width and nvert are loaded before the plane barrier so
 // their latency overlaps the velocity conversion of the next plane.
 constexpr int EDDY_BX = 32, EDDY_BY = 8, EDDY_PX = EDDY_BX + 2, EDDY_PN = EDDY_PX * (EDDY_BY + 2);
-static __global__ void __launch_bounds__(EDDY_BX *EDDY_BY, 4)
-    eddy_viscosity_kernel(const DevCfg c, const double *const *qu, const double *const *met, const double *aj,
-                          const double *delta2, const double *nvert, double *nut, int kchunk,
-                          const double *const *qn = nullptr, const double *csp = nullptr) {
-  __shared__ double us[3][3][EDDY_PN];  // [slot][component][node]
-  __shared__ double stq[4][EDDY_PN];    // raw rho, rhoU, rhoV, rhoW of the plane in flight
-  __shared__ unsigned char stv[EDDY_PN];  // the staged node's velocity source: 0 none, 1 qu, 2 qn
-  pdl_wait();
+struct EddySmem {
+  double us[3][3][EDDY_PN];   // [slot][component][node]
+  double stq[4][EDDY_PN];     // raw rho, rhoU, rhoV, rhoW of the plane in flight
+  unsigned char stv[EDDY_PN];  // the staged node's velocity source: 0 none, 1 qu, 2 qn
+  int again;                  // a quotient out of the branch-free ones' range: the column is done again
+};
+template <bool IEEE>
+__device__ __forceinline__ void eddy_march(EddySmem &es, const DevCfg &c, const double *const *qu, const double *const *met,
+                                           const double *aj, const double *delta2, const double *nvert, double *nut,
+                                           int kchunk, const double *const *qn, const double *csp) {
+  auto &us = es.us;
+  auto &stq = es.stq;
+  auto &stv = es.stv;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * EDDY_BX + tx;
   const int i0 = 1 + blockIdx.x * EDDY_BX, j0 = 1 + blockIdx.y * EDDY_BY;
   const int kb = 1 + blockIdx.z * kchunk, ke = min(c.mz - 1, kb + kchunk);
@@ -621,12 +626,14 @@ static __global__ void __launch_bounds__(EDDY_BX *EDDY_BY, 4)
     for (int e = tid; e < EDDY_PN; e += EDDY_BX * EDDY_BY) {
       double u0 = 0., u1 = 0., u2 = 0.;
       if (stv[e]) {
-        const Den<double> r(stq[0][e]);
+        const DenOf<double, IEEE> r(stq[0][e]);
+        const double u[3] = {r(stq[1][e]), r(stq[2][e]), r(stq[3][e])};
+        if (!IEEE && mag_hi(stq[0][e]) >= mag_pow2(960)) es.again = 1;
         // lUcat x = 0 with -twoD 1 (rhs.c:1349), except where the dynamic
         // model rewrote it from the state (les.c:255)
-        u0 = (c.twod == 1 && stv[e] == 1) ? 0. : r(stq[1][e]);
-        u1 = r(stq[2][e]);
-        u2 = r(stq[3][e]);
+        u0 = (c.twod == 1 && stv[e] == 1) ? 0. : u[0];
+        u1 = u[1];
+        u2 = u[2];
       }
       us[s][0][e] = u0;
       us[s][1][e] = u1;
@@ -688,10 +695,27 @@ static __global__ void __launch_bounds__(EDDY_BX *EDDY_BY, 4)
         const double Szz = 0.5 * (g[2][2] + g[2][2]) - Sdd;
         const double Sabs = sqrt(2.0 * (Sxx * Sxx + Sxy * Sxy + Sxz * Sxz + Sxy * Sxy + Syy * Syy + Syz * Syz +
                                         Sxz * Sxz + Syz * Syz + Szz * Szz));
-        nut[n] = cs * d2 * Sabs;  // CS * pow(pow(1/aj,1/3),2) * |S|
+        if (!IEEE && !finite_hi(Sabs)) es.again = 1;  // (as a quotient out of range leaves it)
+        nut[n] = cs * d2 * Sabs;                      // CS * pow(pow(1/aj,1/3),2) * |S|
       }
     }
   }
+}
+static __device__ __noinline__ void eddy_again(EddySmem &es, const DevCfg &c, const double *const *qu,
+                                               const double *const *met, const double *aj, const double *delta2,
+                                               const double *nvert, double *nut, int kchunk, const double *const *qn,
+                                               const double *csp) {
+  eddy_march<true>(es, c, qu, met, aj, delta2, nvert, nut, kchunk, qn, csp);
+}
+static __global__ void __launch_bounds__(EDDY_BX *EDDY_BY, 4)
+    eddy_viscosity_kernel(const __grid_constant__ DevCfg c, const double *const *qu, const double *const *met,
+                          const double *aj, const double *delta2, const double *nvert, double *nut, int kchunk,
+                          const double *const *qn = nullptr, const double *csp = nullptr) {
+  __shared__ EddySmem es;
+  if (threadIdx.x == 0 && threadIdx.y == 0) es.again = 0;  // (a barrier follows ahead of the first quotient)
+  pdl_wait();
+  eddy_march<false>(es, c, qu, met, aj, delta2, nvert, nut, kchunk, qn, csp);
+  if (__syncthreads_or(es.again)) eddy_again(es, c, qu, met, aj, delta2, nvert, nut, kchunk, qn, csp);
 }
 // (32^3 FP64: 16.9 us per launch with chunks of at least four planes and a
 // quotient chain per node, 7.7 with chunks from one plane and cb_div.cuh)
@@ -731,7 +755,7 @@ static inline dim3 eddy_grid(const DevCfg &c, int kchunk) {
 // curvature rule with y = z = min(y, z).  Boundary nodes keep (s_x, s_y, s_z).
 __device__ __forceinline__ double sensor_ri(double fR, double f0, double fL, double ks) {
   const double dfL = fL - f0, dfR = f0 - fR;
-  return Den<double>(dfL * dfL + dfR * dfR + ks)(fabs(2 * dfL * dfR) + ks);
+  return quot(fabs(2 * dfL * dfR) + ks, dfL * dfL + dfR * dfR + ks);
 }
 __device__ __forceinline__ double sensor_ramp(double fL, double f0, double fR, double fRR, double ks) {
   const double rL = sensor_ri(fL, f0, fR, ks), rR = sensor_ri(f0, fR, fRR, ks);
@@ -742,7 +766,7 @@ __device__ __forceinline__ double sensor_ramp(double fL, double f0, double fR, d
 }
 __device__ __forceinline__ double eos_node(const DevCfg &c, const double *const *q, long long n) {
   const double r = q[0][n];
-  return r != 0.0 ? (c.gamma - 1) * (q[4][n] - Den<double>(r)(0.5 * (q[1][n] * q[1][n] + q[2][n] * q[2][n] + q[3][n] * q[3][n])))
+  return r != 0.0 ? (c.gamma - 1) * (q[4][n] - quot(0.5 * (q[1][n] * q[1][n] + q[2][n] * q[2][n] + q[3][n] * q[3][n]), r))
                   : 0.0;
 }
 __device__ __forceinline__ double pmin(double a, double b) { return (a < b) ? a : b; }

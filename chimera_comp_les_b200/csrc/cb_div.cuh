@@ -32,7 +32,9 @@
 // overflow is tested there; a tile march that met one out of bounds is done
 // again with a / b and sqrt (FLUX_IEEE).  The bounds on the nodes leave room for
 // everything the faces build from them: squared WENO smoothness measures stay
-// below 2^960, their weights and sums above 2^-960.
+// below 2^960, their weights and sums above 2^-960.  The model's kernels test their
+// results, where a NaN of a quotient shows, and the denominators' upper end, and
+// form them again with a / b; the sensor takes quot.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -171,6 +173,11 @@ __device__ __forceinline__ float root(float x) {
   return g;
 }
 
+template <bool IEEE>
+__device__ __forceinline__ double by27(double a) {
+  if constexpr (IEEE) return plain_quot(a, 27.0);
+  else return Den<double>(27.0, 1.0 / 27.0)(a);
+}
 template <typename R, bool IEEE>
 __device__ __forceinline__ R root_of(R x) {
   if constexpr (IEEE) return plain_root(x);
@@ -188,6 +195,13 @@ __host__ __device__ constexpr unsigned mag_pow2(int e) { return (unsigned)(1023 
 // |b| in 2^-960 .. 2^960
 __device__ __forceinline__ bool in_range(double b) {
   return mag_hi(b) - mag_pow2(-960) < mag_pow2(960) - mag_pow2(-960);
+}
+
+// a / b as the branch-free quotient, redone by a / b where that leaves its range
+// (an infinite or overflowing quotient included)
+__device__ __forceinline__ double quot(double a, double b) {
+  const double q = Den<double>(b)(a);
+  return mag_hi(b) < mag_pow2(960) && finite_hi(q) ? q : a / b;
 }
 
 // Whether a node's conserved state v and pressure p lie outside |x| < 2^230,

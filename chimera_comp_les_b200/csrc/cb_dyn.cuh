@@ -25,20 +25,34 @@ __device__ __forceinline__ bool dyn_interior(const DevCfg &c, int i, int j, int 
   return i >= 1 && i <= c.mx - 2 && j >= 1 && j <= c.my - 2 && k >= 1 && k <= c.mz - 2;
 }
 
-// the three components at once: they share the density's reciprocal
+// the three components at once: they share the density's reciprocal.  IEEE: by
+// a / b; else top collects the densities' magnitudes, for top_out below.
+template <bool IEEE>
 __device__ __forceinline__ void dyn_u(const DevCfg &c, const double *const *q, const double *const *qu,
-                                      const double *nvert, int i, int j, int k, bool reached, double u[3]) {
+                                      const double *nvert, int i, int j, int k, bool reached, double u[3], unsigned &top) {
   const long long m = gidx(c, i, j, k);
   const bool cur = reached && dyn_interior(c, i, j, k) && nvert[m] <= 1.1;  // les.c:255, x kept
   const double *const *s = cur ? q : qu;
   u[0] = u[1] = u[2] = 0.0;
   if (!s) return;
-  const Den<double> r(s[0][m]);
-  // the last CalcUCat's x is 0 with -twoD 1 (rhs.c:1349)
-  if (cur || c.twod != 1) u[0] = r(s[1][m]);
-  u[1] = r(s[2][m]);
-  u[2] = r(s[3][m]);
+  const double rho = s[0][m];
+  const bool x0 = !cur && c.twod == 1;  // the last CalcUCat's x is 0 with -twoD 1 (rhs.c:1349)
+  if constexpr (IEEE) {
+    if (!x0) u[0] = s[1][m] / rho;
+    u[1] = s[2][m] / rho;
+    u[2] = s[3][m] / rho;
+  } else {
+    top = max(top, mag_hi(rho));
+    const Den<double> r(rho);
+    if (!x0) u[0] = r(s[1][m]);
+    u[1] = r(s[2][m]);
+    u[2] = r(s[3][m]);
+  }
 }
+// Denominators beyond the branch-free quotients' upper end.  Below their lower
+// end, and for an infinite numerator or quotient, the quotient is not finite,
+// nor is the result it enters, which the callers test.
+__device__ __forceinline__ bool top_out(unsigned top) { return top >= mag_pow2(960); }
 
 __device__ __forceinline__ void dyn_node(const DevCfg &c, long long t, int &i, int &j, int &k) {
   const unsigned u = (unsigned)t, px = (unsigned)c.px, py = (unsigned)c.py;
@@ -50,7 +64,7 @@ __device__ __forceinline__ void dyn_node(const DevCfg &c, long long t, int &i, i
 
 // (1) velocity gradients (du/dx .. dw/dz) and |S| at interior nodes with
 // nvert <= 1.1 (les.c:234-284); zero on every other node of the padded box.
-static __global__ void dyn_grad_kernel(const DevCfg c, const double *const *q, const double *const *qu,
+static __global__ void __launch_bounds__(256, 4) dyn_grad_kernel(const DevCfg c, const double *const *q, const double *const *qu,
                                        const double *const *met, const double *aj, const double *nvert,
                                        double *const *A, double *Sabs) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < c.plane; t += (long long)gridDim.x * blockDim.x) {
@@ -60,14 +74,26 @@ static __global__ void dyn_grad_kernel(const DevCfg c, const double *const *q, c
     double sabs = 0.;
     if (i <= c.mx + 1 && j <= c.my + 1 && dyn_interior(c, i, j, k) && nvert[t] <= 1.1) {
       double d[3][3];
+      unsigned top = 0;
 #pragma unroll
       for (int x = 0; x < 3; x++) {
         const int di = x == 0, dj = x == 1, dk = x == 2;
         double up[3], um[3];
-        dyn_u(c, q, qu, nvert, i + di, j + dj, k + dk, false, up);
-        dyn_u(c, q, qu, nvert, i - di, j - dj, k - dk, true, um);
+        dyn_u<false>(c, q, qu, nvert, i + di, j + dj, k + dk, false, up, top);
+        dyn_u<false>(c, q, qu, nvert, i - di, j - dj, k - dk, true, um, top);
 #pragma unroll
         for (int a = 0; a < 3; a++) d[a][x] = (up[a] - um[a]) * 0.5;
+      }
+      if (top_out(top) || !finite_hi(d[0][0] + d[0][1] + d[0][2] + d[1][0] + d[1][1] + d[1][2] + d[2][0] + d[2][1] + d[2][2])) {
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+          const int di = x == 0, dj = x == 1, dk = x == 2;
+          double up[3], um[3];
+          dyn_u<true>(c, q, qu, nvert, i + di, j + dj, k + dk, false, up, top);
+          dyn_u<true>(c, q, qu, nvert, i - di, j - dj, k - dk, true, um, top);
+#pragma unroll
+          for (int a = 0; a < 3; a++) d[a][x] = (up[a] - um[a]) * 0.5;
+        }
       }
       const double ajc = aj[t];
 #pragma unroll
@@ -134,11 +160,11 @@ static __global__ void dyn_copy_kernel(const DevCfg c, double *const *f, int npl
 // formed here once per node.
 constexpr int DYN_BX = 32, DYN_BY = 6, DYN_PX = DYN_BX + 2, DYN_PN = DYN_PX * (DYN_BY + 2), DYN_NF = 14;
 constexpr size_t DYN_LM_SMEM = sizeof(double) * 2 * DYN_NF * DYN_PN;
-static __global__ void __launch_bounds__(DYN_BX *DYN_BY, 2)
-    dyn_lm_tiled_kernel(const DevCfg c, const double *const *q, const double *const *qu, const double *aj,
-                        const double *nvert, const double *const *A, const double *Sabs, double *LM, double *MM,
-                        int kchunk, double tf_mult, int scale27) {
-  extern __shared__ double dsm[];  // [slot][field][node]
+template <bool IEEE>
+__device__ __forceinline__ void dyn_lm_march(const DevCfg &c, const double *const *q, const double *const *qu,
+                                             const double *aj, const double *nvert, const double *const *A,
+                                             const double *Sabs, double *LM, double *MM, int kchunk, double tf_mult,
+                                             int scale27, double *dsm, int *again) {  // dsm: [slot][field][node]
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * DYN_BX + tx;
   const int i0 = 1 + blockIdx.x * DYN_BX, j0 = 1 + blockIdx.y * DYN_BY;
   const int kb = 1 + blockIdx.z * kchunk, ke = min(c.mz - 1, kb + kchunk);
@@ -154,7 +180,8 @@ static __global__ void __launch_bounds__(DYN_BX *DYN_BY, 2)
       for (int f = 0; f < DYN_NF; f++) v[f] = 0.;
       if (xi <= c.mx - 1 && yj <= c.my - 1) {
         const long long m = gidx(c, xi, yj, kk);
-        dyn_u(c, q, qu, nvert, xi, yj, kk, true, v);
+        unsigned top = 0;  // (not tested here: the filtered density below holds at least 1/64 of each)
+        dyn_u<IEEE>(c, q, qu, nvert, xi, yj, kk, true, v, top);
         v[3] = q[0][m]; v[4] = q[1][m]; v[5] = q[2][m]; v[6] = q[3][m];
         v[7] = 0.5 * (A[0][m] + A[0][m]); v[8] = 0.5 * (A[1][m] + A[3][m]); v[9] = 0.5 * (A[2][m] + A[6][m]);
         v[10] = 0.5 * (A[4][m] + A[4][m]); v[11] = 0.5 * (A[5][m] + A[7][m]); v[12] = 0.5 * (A[8][m] + A[8][m]);
@@ -214,7 +241,7 @@ static __global__ void __launch_bounds__(DYN_BX *DYN_BY, 2)
         // the weights sum to 8: dividing by the sum is the exact scaling by 1/8
         const double rws = 0.125;
         const double _rho = f[0] * rws, _rhou = f[1] * rws, _rhov = f[2] * rws, _rhow = f[3] * rws;
-        const Den<double> drho(_rho);
+        const DenOf<double, IEEE> drho(_rho);
         const int sym[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
         const int prod[3][3] = {{4, 5, 6}, {5, 7, 8}, {6, 8, 9}};
         const double fr[3] = {_rhou, _rhov, _rhow};
@@ -247,9 +274,9 @@ static __global__ void __launch_bounds__(DYN_BX *DYN_BY, 2)
                      2.0 * f2 * (SSh[a][b] * Sx[a][b] - 0.33 * SSh[a][a] * Sx[b][b]);
             L_cat += Lij[a][b] * Sx[a][b] - 0.33 * Sx[a][a] * Lij[b][b];
           }
-        const Den<double> d27(27.0, 1.0 / 27.0);
-        lm = scale27 ? d27(L_cat) : L_cat;
-        mm = scale27 ? d27(M_cat) : M_cat;
+        lm = scale27 ? by27<IEEE>(L_cat) : L_cat;
+        mm = scale27 ? by27<IEEE>(M_cat) : M_cat;
+        if (!IEEE && (mag_hi(_rho) >= mag_pow2(950) || !finite_hi(lm + mm))) *again = 1;
       }
       LM[n] = lm;
       MM[n] = mm;
@@ -259,6 +286,24 @@ static __global__ void __launch_bounds__(DYN_BX *DYN_BY, 2)
 #pragma unroll
     for (int x = 0; x < 6; x++) Sc[x] = Sn[x];
   }
+}
+static __device__ __noinline__ void dyn_lm_again(const DevCfg &c, const double *const *q, const double *const *qu,
+                                                 const double *aj, const double *nvert, const double *const *A,
+                                                 const double *Sabs, double *LM, double *MM, int kchunk, double tf_mult,
+                                                 int scale27) {
+  extern __shared__ double dsm[];
+  dyn_lm_march<true>(c, q, qu, aj, nvert, A, Sabs, LM, MM, kchunk, tf_mult, scale27, dsm, nullptr);
+}
+static __global__ void __launch_bounds__(DYN_BX *DYN_BY, 2)
+    dyn_lm_tiled_kernel(const __grid_constant__ DevCfg c, const double *const *q, const double *const *qu, const double *aj,
+                        const double *nvert, const double *const *A, const double *Sabs, double *LM, double *MM,
+                        int kchunk, double tf_mult, int scale27) {
+  extern __shared__ double dsm[];
+  __shared__ int again;
+  if (threadIdx.x == 0 && threadIdx.y == 0) again = 0;
+  __syncthreads();
+  dyn_lm_march<false>(c, q, qu, aj, nvert, A, Sabs, LM, MM, kchunk, tf_mult, scale27, dsm, &again);
+  if (__syncthreads_or(again)) dyn_lm_again(c, q, qu, aj, nvert, A, Sabs, LM, MM, kchunk, tf_mult, scale27);
 }
 
 // (3) Cs from the 27-node means of LM and MM at interior nodes
@@ -432,6 +477,7 @@ static __global__ void dyn_avg_kernel(const DevCfg c, const double *aj, const do
     const long long n = gidx(c, i, j, k);
     if (!(nvert[n] < 0.1)) continue;
     double vs = 0.0, ws = 0.0;
+    int top = 0;  // aj's high words (aj > 0)
 #pragma unroll
     for (int R = 0; R < 3; R++)
 #pragma unroll
@@ -439,10 +485,21 @@ static __global__ void dyn_avg_kernel(const DevCfg c, const double *aj, const do
 #pragma unroll
         for (int P = 0; P < 3; P++) {
           const long long m = gidx(c, i + P - 1, j + Q - 1, k + R - 1);
+          top = max(top, __double2hiint(aj[m]));
           const double w = Den<double>(aj[m])(1.);
           vs += w * ct[m];
           ws += w;
         }
+    if (top_out((unsigned)top << 1) || !finite_hi(vs + ws)) {
+      vs = ws = 0.0;
+#pragma unroll 1
+      for (int x = 0; x < 27; x++) {
+        const long long m = gidx(c, i + x % 3 - 1, j + x / 3 % 3 - 1, k + x / 9 - 1);
+        const double w = 1. / aj[m];
+        vs += w * ct[m];
+        ws += w;
+      }
+    }
     cs[n] = vs / ws;
   }
 }

@@ -18,6 +18,7 @@ N = (40, 17, 18)  # two tiles in i, three to four in j
 SCHEMES = {
     "muscl": dict(les=1, fluxorder=2, s_x=0.0, s_y=0.0, s_z=0.0),
     "muscl_roe": dict(les=0, fluxorder=2, flux=1, inviscid=1),
+    "first_blend": dict(les=1, fluxorder=1, s_x=0.5, s_y=0.5, s_z=0.5),
     "weno3_blend": dict(les=1, fluxorder=3, s_x=0.5, s_y=0.5, s_z=0.5),
     "weno3_roe": dict(les=1, fluxorder=3, flux=1, s_x=0.0, s_y=0.0, s_z=0.0),
     "std_weno3": dict(les=0, fluxorder=3),
@@ -30,7 +31,7 @@ SCHEMES = {
 DT = {"jump": 1e-20, "dense": 1e-150, "dense_even": 1e-150}
 CASES = ([(s, f"jump{a}") for s in ("weno3_blend", "weno3_roe", "std_weno3", "weno5", "weno5_roe") for a in (0, 1, 2)]
          + [(s, f"ramp{a}") for s in ("weno3_roe", "weno5") for a in (0, 1)]
-         + [(s, "dense") for s in ("muscl", "muscl_roe")]
+         + [(s, "dense") for s in ("muscl", "muscl_roe", "first_blend")]
          + [(s, "dense_even") for s in ("weno3_blend", "weno3_roe", "std_weno3", "central", "central_two_point")]
          + [(s, "subnormal") for s in ("muscl_roe", "std_weno3", "weno5_roe", "central_two_point")])
 
@@ -108,3 +109,62 @@ def test_fp64_matches_the_restatement(scheme, kind, body):
             b.SetInitialCondition(q)
             b.RungeKutta(1)
             assert _worst(b.Q(), ref["q_steps"], far) <= RTOL_L2
+
+
+# ------------------------------------------- model and sensor kernels -------
+def _momentum(shape, rho, u):
+    """Density rho (scaled to its maximum) and velocities of size u; energy 1."""
+    q = W.random_smooth_state(shape, seed=9)
+    r = rho * (q[..., :1] / q[..., :1].max())
+    return np.concatenate([r, r * (u * q[..., 1:4]), q[..., 4:]], axis=-1)
+
+
+@pytest.mark.parametrize("les", [1, 2])
+@pytest.mark.parametrize("rho,scale", [(8e307, 1.0), (1e-310, 1.0), (1.0, 8.2e-103)], ids=["dense", "subnormal", "fine_grid"])
+def test_eddy_viscosity_beyond_the_quotients_range(les, rho, scale):
+    """nu_t and the dynamic coefficient; fine_grid: 1 / aj of aj above 2^1022."""
+    coords = scale * W.periodic_grid(N, 2 * np.pi, amp=0.01)
+    shape = coords.shape[:3]
+    cfg = O.Config(mx=N[0] + 2, my=N[1] + 2, mz=N[2] + 2, ren=500.0, ma=0.3, pr=0.71, inviscid=0, les=les, max_cs=0.1)
+    if les == 2 and rho > 1e300:
+        pytest.skip("the test filter's sum of densities overflows in the reference too")
+    q = _momentum(shape, rho, 0.3)
+    with np.errstate(all="ignore"):
+        ref = oracle_run(cfg, coords, q, np.zeros(shape))
+    if scale != 1.0:
+        assert ref["metrics"]["aj"].min() > 2.0 ** 1022
+    with gpu_block(cfg) as b:
+        b.FormMetrics(coords)
+        b.SetInitialCondition(q)
+        b.CalcUCat()
+        b.Compute_eddy_viscosity_LES()
+        nut = b.nu_t()
+        cs = b.CS() if les == 2 else None
+    assert np.isfinite(ref["nut"]).all() and ref["nut"].max() > 0.0
+    assert np.abs(nut - ref["nut"]).max() <= RTOL_L2 * ref["nut"].max()
+    if les == 2:
+        assert np.abs(cs - ref["cs"]).max() <= RTOL_L2 * ref["cs"].max()
+
+
+@pytest.mark.parametrize("kind", ["jump", "dense"])
+def test_sensor_beyond_the_quotients_range(kind):
+    """jump: a pressure jump of 1e160, whose square overflows on one side; dense: the EOS of densities above 2^1022."""
+    coords = W.periodic_grid(N, 2 * np.pi, amp=0.04)
+    shape = coords.shape[:3]
+    cfg = O.Config(mx=N[0] + 2, my=N[1] + 2, mz=N[2] + 2, ma=0.3, pr=0.71, inviscid=1, les=1, fluxorder=2, calc_sigma=1,
+                   s_x=1.0, s_y=1.0, s_z=1.0)
+    far = None
+    if kind == "jump":
+        q = W.random_smooth_state(shape, seed=9)
+        far = np.zeros(shape, bool)
+        far[:, :, shape[2] // 3:2 * shape[2] // 3] = True
+        q[far] = [1.0, 0.3, -0.2, 0.1, 1e160]
+    else:
+        q, far = _state(shape, "dense")
+    with np.errstate(all="ignore"):
+        ref = oracle_run(cfg, coords, q, np.zeros(shape))["rhs"]
+    assert np.isfinite(ref).all()
+    with gpu_block(cfg) as b:
+        b.FormMetrics(coords)
+        b.SetInitialCondition(q)
+        assert _worst(b.formRHS(0), ref, far) <= RTOL_L2
