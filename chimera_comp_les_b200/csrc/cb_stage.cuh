@@ -1342,6 +1342,9 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
   constexpr bool SMET = StageMet<MIX, NV0, FLUX>::on;
   constexpr int MPX = RG::MPX, MPN = RG::MPN;
   constexpr bool PLAIN = (FLUX & FLUX_PLAIN) != 0;
+  // a step without WENO weights squares no value: beyond the density, a value out
+  // of bounds shows in the fluxes or in the status of the new state
+  constexpr bool LEAN = !RHS_MODE && PLAIN && ((FLUX & (FLUX_W3 | FLUX_W5)) == 0 || (LES && (FLUX & FLUX_SIGMA1) != 0));
   double *stg = smem_d;  // [NSTG][PN] raw FP64 Q, nvert and carried pressure of the next plane
   float4 *mts = reinterpret_cast<float4 *>(smem_d + (size_t)NSTG * PN);  // [3][MPN] metric slot (SMET)
   double *nts = reinterpret_cast<double *>(mts + (SMET ? 3 * MPN : 0));   // [MPN] nu_t slot (SMET)
@@ -1421,7 +1424,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
           v[F_V] = rho(v[2]);
           v[F_W] = rho(v[3]);
           v[F_T] = rho(v[F_P]);
-          if (!IEEE && wide_state(v, v[F_P])) *Rg.wd = 1;
+          if (!IEEE && (LEAN ? !in_range(r) : wide_state(v, v[F_P]))) *Rg.wd = 1;
         }
         if (MIX) {
           v[F_RE] -= c.e_ref;
