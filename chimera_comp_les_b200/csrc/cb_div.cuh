@@ -57,19 +57,17 @@ __device__ __forceinline__ double rsqrt_approx(double b) {
 // |b| < 2^126 it has the bits of the fast division the form is compiled with
 // (-prec-div=false; none of 1.6e9 random pairs with exponents up to +-120
 // differed, nor 1 / b, nor the square root), without that division's range
-// scaling; a larger or infinite b gives 0.  The denominators here are
-// densities, squared WENO smoothness measures (at least 1e-12) and sums of
-// weights.  Measured per step:
-// WENO5-JS + Roe 192^3 7.8 -> 5.9 ms, immersed sphere 96x96x128 1.91 -> 1.63 ms.
+// scaling.  rcp_approx flushes: a larger b gives 0, a subnormal one infinity.  It
+// serves the WENO weights, scaled so that no finite squared smoothness measure
+// reaches 2^126, and the sum of two roots.  Densities and Roe's c^2 take 1 / b,
+// and the roots sqrtf and rsqrtf: the full-range approximations (squared metrics
+// are subnormal where a cell face is smaller than 1e-19).  Measured per step, with
+// every quotient flushing: WENO5-JS + Roe 192^3 7.8 -> 5.9 ms, immersed sphere
+// 96x96x128 1.91 -> 1.63 ms; the full-range ones take back 1.4 and 1.9 % (MUSCL
+// 128^3 0.8 %).
 __device__ __forceinline__ float rcp_approx(float b) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-  return y;
-}
-
-__device__ __forceinline__ float rsqrt_approx(float b) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
   return y;
 }
 
@@ -113,7 +111,7 @@ struct Den;
 template <>
 struct Den<float> {
   float y;
-  __device__ __forceinline__ explicit Den(float b) : y(rcp_approx(b)) {}
+  __device__ __forceinline__ explicit Den(float b) : y(1.f / b) {}
   __device__ __forceinline__ Den(float, float y_) : y(y_) {}
   __device__ __forceinline__ Den doubled() const { return Den(0.f, 0.5f * y); }  // divides by 2 b
   // __fmul_rn: the quotient is rounded before it enters a sum
@@ -135,6 +133,18 @@ struct Den<double> {
   }
 };
 
+// A denominator that is well inside the range: FP32 by the flushing reciprocal.
+template <typename R>
+struct FlushDen : Den<R> {
+  using Den<R>::Den;
+};
+template <>
+struct FlushDen<float> {
+  float y;
+  __device__ __forceinline__ explicit FlushDen(float b) : y(rcp_approx(b)) {}
+  __device__ __forceinline__ float operator()(float a) const { return __fmul_rn(a, y); }
+};
+
 // The same by a / b: for values out of the branch-free quotients' range.  Out of
 // line, for code that hardly ever runs.
 template <typename R>
@@ -150,6 +160,8 @@ struct PlainDen {
 };
 template <typename R, bool IEEE>
 using DenOf = std::conditional_t<IEEE, PlainDen<R>, Den<R>>;
+template <typename R, bool IEEE>
+using FlushDenOf = std::conditional_t<IEEE, PlainDen<R>, FlushDen<R>>;
 
 // a / 3 (FP64: with the reciprocal rounded to nearest)
 template <typename R, bool IEEE>
@@ -167,11 +179,7 @@ __device__ __forceinline__ double root(double x) {
   h = fma(h, s, h);
   return fma(fma(-g, g, x), h, g);
 }
-__device__ __forceinline__ float root(float x) {
-  float g;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(x));
-  return g;
-}
+__device__ __forceinline__ float root(float x) { return sqrtf(x); }
 
 template <bool IEEE>
 __device__ __forceinline__ double by27(double a) {

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(EF_BX *EF_BY)
     for (int e = tid; e < EF_PN; e += EF_BX * EF_BY) {
       float u0 = 0.f, u1 = 0.f, u2 = 0.f;
       if (stv[e]) {
-        const float ri = rcp_approx((float)stq[0][e]);
+        const float ri = 1.f / (float)stq[0][e];
         u0 = c.twod == 1 ? 0.f : (float)stq[1][e] * ri;  // lUcat x = 0 with -twoD 1 (rhs.c:1349)
         u1 = (float)stq[2][e] * ri;
         u2 = (float)stq[3][e] * ri;

@@ -278,20 +278,25 @@ template <typename R>
 __device__ __forceinline__ R muscl_l(R qm, R q0, R qp) { return q0 + R(0.5) * r_minmod(qp - q0, q0 - qm); }
 template <typename R>
 __device__ __forceinline__ R muscl_r(R qm, R q0, R qp) { return q0 - R(0.5) * r_minmod(qp - q0, q0 - qm); }
-template <typename R, class D = Den<R>>
+// WENO3.  FP32: the slopes halved and eps quartered, which scales the squared
+// smoothness measures by exactly 1/16 and cancels in the weights: a measure
+// above 2^126, whose reciprocal would be flushed, stays below it.
+template <typename R>
+constexpr R WENO_HALF = sizeof(R) == 4 ? R(0.5) : R(1);
+template <typename R, class D = FlushDen<R>>
 __device__ __forceinline__ R weno3_l(R qm, R q0, R qp) {
-  const R d0 = R(0.6666667), d1 = R(0.3333333), eps = R(1e-6);  // rhs.c:2386 (truncated weights)
+  const R d0 = R(0.6666667), d1 = R(0.3333333), h = WENO_HALF<R>, eps = R(1e-6) * h * h;  // rhs.c:2386 (truncated weights)
   R r0 = R(0.5) * q0 + R(0.5) * qp, r1 = R(-0.5) * qm + R(1.5) * q0;
-  R b0 = (qp - q0) * (qp - q0), b1 = (qm - q0) * (qm - q0);
+  const R e0 = h * (qp - q0), e1 = h * (qm - q0), b0 = e0 * e0, b1 = e1 * e1;
   const R a0 = D((eps + b0) * (eps + b0))(d0), a1 = D((eps + b1) * (eps + b1))(d1);
   const D as(a0 + a1);
   return as(a0) * r0 + as(a1) * r1;
 }
-template <typename R, class D = Den<R>>
+template <typename R, class D = FlushDen<R>>
 __device__ __forceinline__ R weno3_r(R qm, R q0, R qp) {
-  const R d0 = R(0.6666667), d1 = R(0.3333333), eps = R(1e-6);
+  const R d0 = R(0.6666667), d1 = R(0.3333333), h = WENO_HALF<R>, eps = R(1e-6) * h * h;
   R r0 = R(1.5) * q0 - R(0.5) * qp, r1 = R(0.5) * qm + R(0.5) * q0;
-  R b0 = (qp - q0) * (qp - q0), b1 = (qm - q0) * (qm - q0);
+  const R e0 = h * (qp - q0), e1 = h * (qm - q0), b0 = e0 * e0, b1 = e1 * e1;
   const R a0 = D((eps + b0) * (eps + b0))(d0), a1 = D((eps + b1) * (eps + b1))(d1);
   const D as(a0 + a1);
   return as(a0) * r0 + as(a1) * r1;
@@ -314,7 +319,7 @@ __device__ __forceinline__ R eno_l(R qm, R q0, R qp, int k) {
 // eps = 1e-6, value sum(alpha_k q_k) / (6 sum(alpha_k)).  The right-biased
 // value at x_{i+1/2} is weno5(v_{i+3}, .., v_{i-1}).  Same operation order as
 // the oracle's restatement (bit-identical in the FP64 form).
-template <typename R, class D = Den<R>>
+template <typename R, class D = FlushDen<R>>
 __device__ __forceinline__ R weno5(R a, R b, R c, R d, R e) {
   const R eps = R(1e-6), c13 = R(13.0 / 12.0);
   const R q0 = (R(2.0) * a - R(7.0) * b) + R(11.0) * c;
@@ -351,39 +356,44 @@ __device__ __forceinline__ void muscl_2(float2 q0, float2 q1, float2 q2, float2 
 // The mixed form's reconstructions of two fields at once.  The multiply-adds
 // are those the compiler forms from weno5 / weno3_l / weno3_r with FP32
 // contraction on (found by comparing every alternative bit for bit), so the
-// values are the scalar functions' own.
+// values are the scalar functions' own.  As in WENO3 above, powers of two keep a
+// finite squared smoothness measure below 2^126: beta and eps are halved, which
+// scales the reciprocals by exactly 4, and the candidates quartered, so that the
+// sums keep their size.  (One finite measure above 2^125 beside two that
+// overflow still gives NaN.)
 __device__ __forceinline__ float2 weno5_2(float2 a, float2 b, float2 c, float2 d, float2 e) {
-  const float c13 = float(13.0 / 12.0);
-  const float2 eps = both(1e-6f), c2 = add2(c, c), c3 = mul2(3.f, c);
-  const float2 q0 = fma2(11.f, c, fma2(-7.f, b, add2(a, a)));
-  const float2 q1 = fma2(2.f, d, fma2(5.f, c, mul2(-1.f, b)));
-  const float2 q2 = sub2(fma2(5.f, d, c2), e);
+  const float c13 = 0.5f * float(13.0 / 12.0);
+  const float2 eps = both(0.5f * 1e-6f), c3 = mul2(3.f, c);
+  const float2 q0 = fma2(2.75f, c, fma2(-1.75f, b, mul2(0.5f, a)));
+  const float2 q1 = fma2(0.5f, d, fma2(1.25f, c, mul2(-0.25f, b)));
+  const float2 q2 = fma2(-0.25f, e, fma2(1.25f, d, mul2(0.5f, c)));
   const float2 t0 = add2(fma2(-2.f, b, a), c), u0 = add2(fma2(-4.f, b, a), c3);
   const float2 t1 = add2(fma2(-2.f, c, b), d), u1 = sub2(b, d);
   const float2 t2 = add2(fma2(-2.f, d, c), e), u2 = add2(fma2(-4.f, d, c3), e);
-  const float2 s0 = add2(eps, fma2(c13, mul2(t0, t0), mul2(0.25f, mul2(u0, u0))));
-  const float2 s1 = add2(eps, fma2(0.25f, mul2(u1, u1), mul2(c13, mul2(t1, t1))));
-  const float2 s2 = add2(eps, fma2(c13, mul2(t2, t2), mul2(0.25f, mul2(u2, u2))));
+  const float2 s0 = add2(eps, fma2(c13, mul2(t0, t0), mul2(0.125f, mul2(u0, u0))));
+  const float2 s1 = add2(eps, fma2(0.125f, mul2(u1, u1), mul2(c13, mul2(t1, t1))));
+  const float2 s2 = add2(eps, fma2(c13, mul2(t2, t2), mul2(0.125f, mul2(u2, u2))));
   const float2 a0 = mul2(0.1f, rcp2(mul2(s0, s0)));
   const float2 a1 = mul2(0.6f, rcp2(mul2(s1, s1)));
   const float2 a2 = mul2(0.3f, rcp2(mul2(s2, s2)));
   const float2 num = fma2(a2, q2, fma2(a0, q0, mul2(a1, q1)));
-  return mul2(num, rcp2(mul2(6.f, add2(add2(a0, a1), a2))));
+  return mul2(num, rcp2(mul2(1.5f, add2(add2(a0, a1), a2))));
 }
 // weno3_l(q0, q1, q2) and weno3_r(q1, q2, q3): both weigh the middle slope
 __device__ __forceinline__ void weno3_2(float2 q0, float2 q1, float2 q2, float2 q3, float2 &l, float2 &r) {
   const float d0 = float(0.6666667), d1 = float(0.3333333);
-  const float2 eps = both(1e-6f), e0 = sub2(q0, q1), e1 = sub2(q2, q1), e2 = sub2(q3, q2);
+  const float2 h0 = mul2(-0.5f, q0), h1 = mul2(0.5f, q1), h2 = mul2(0.5f, q2), h3 = mul2(-0.5f, q3);
+  const float2 eps = both(0.25f * 1e-6f), e0 = add2(h0, h1), e1 = sub2(h2, h1), e2 = add2(h3, h2);  // halved, either sign
   const float2 s0 = fma2(e0, e0, eps), s1 = fma2(e1, e1, eps), s2 = fma2(e2, e2, eps);
   const float2 y0 = rcp2(mul2(s0, s0)), y1 = rcp2(mul2(s1, s1)), y2 = rcp2(mul2(s2, s2));
   {
     const float2 a0 = mul2(d0, y1), a1 = mul2(d1, y0), y = rcp2(add2(a0, a1));
-    const float2 r0 = fma2(0.5f, q1, mul2(0.5f, q2)), r1 = fma2(1.5f, q1, mul2(-0.5f, q0));
+    const float2 r0 = fma2(0.5f, q1, h2), r1 = fma2(1.5f, q1, h0);
     l = fma2(mul2(a0, y), r0, mul2(mul2(a1, y), r1));
   }
   {
     const float2 a0 = mul2(d0, y2), a1 = mul2(d1, y1), y = rcp2(add2(a0, a1));
-    const float2 r0 = fma2(1.5f, q2, mul2(-0.5f, q3)), r1 = fma2(0.5f, q1, mul2(0.5f, q2));
+    const float2 r0 = fma2(1.5f, q2, h3), r1 = fma2(0.5f, q1, h2);
     r = fma2(mul2(a0, y), r0, mul2(mul2(a1, y), r1));
   }
 }
@@ -429,7 +439,7 @@ __device__ __forceinline__ bool rusanov(const R QL[5], const R QR[5], R pL, R pR
   R uconL, uconR, saL, saR;
   const R gii = h[0] * h[0] + h[1] * h[1] + h[2] * h[2];
   if constexpr (MIX) {
-    const R ril = rcp_approx(QL[0]), rir = rcp_approx(QR[0]);
+    const R ril = R(1) / QL[0], rir = R(1) / QR[0];
     const R UR = (h[0] * QR[1] + h[1] * QR[2] + h[2] * QR[3]) * rir;
     uconL = use_qr_for_l ? UR : (h[0] * QL[1] + h[1] * QL[2] + h[2] * QL[3]) * ril;
     uconR = r_from_l ? uconL : UR;
@@ -481,10 +491,10 @@ __device__ __forceinline__ bool roe(const R QL[5], const R QR[5], R pL, R pR, co
   const R hh = h[0] * h[0] + h[1] * h[1] + h[2] * h[2], area = rt_of(hh);
   const D da(area);
   R ria = R(0);
-  if constexpr (MIX) ria = rsqrt_approx(hh);
+  if constexpr (MIX) ria = rsqrtf(hh);
   const R nx = MIX ? h[0] * ria : da(h[0]), ny = MIX ? h[1] * ria : da(h[1]), nz = MIX ? h[2] * ria : da(h[2]);
   const R sl = rt_of(QL[0]), sr = rt_of(QR[0]);
-  const D ds(sl + sr);
+  const FlushDenOf<R, IEEE> ds(sl + sr);
   const R ris = MIX ? ds(R(1)) : R(0);
   const R wl = MIX ? sl * ris : ds(sl), wr = MIX ? sr * ris : ds(sr);
   const R uL = CB_DIVL(QL[1]), vL = CB_DIVL(QL[2]), zL = CB_DIVL(QL[3]);
@@ -559,7 +569,7 @@ __device__ __forceinline__ bool weno5_face(const DevCfg &c, const DevFields &F, 
       node_qp<R, MIX, IEEE>(c, v, pst, pst ? ldg(F.pin + g) : 0.0, qd, pd, Rg.wd);
     }
   }
-  using D = DenOf<R, IEEE>;
+  using FD = FlushDenOf<R, IEEE>;
   if constexpr (MIX) {  // fields two at a time; the pressure is the energy's partner
 #pragma unroll
     for (int q = 0; q < 6; q += 2) {
@@ -574,11 +584,11 @@ __device__ __forceinline__ bool weno5_face(const DevCfg &c, const DevFields &F, 
   } else {
 #pragma unroll
     for (int q = 0; q < 5; q++) {
-      QL[q] = weno5<R, D>(Qm[q], Q[0][q], Q[1][q], Q[2][q], Q[3][q]);
-      QR[q] = weno5<R, D>(Qp[q], Q[3][q], Q[2][q], Q[1][q], Q[0][q]);
+      QL[q] = weno5<R, FD>(Qm[q], Q[0][q], Q[1][q], Q[2][q], Q[3][q]);
+      QR[q] = weno5<R, FD>(Qp[q], Q[3][q], Q[2][q], Q[1][q], Q[0][q]);
     }
-    pL = weno5<R, D>(Pm, P[0], P[1], P[2], P[3]);
-    pR = weno5<R, D>(Pp, P[3], P[2], P[1], P[0]);
+    pL = weno5<R, FD>(Pm, P[0], P[1], P[2], P[3]);
+    pR = weno5<R, FD>(Pp, P[3], P[2], P[1], P[0]);
   }
   return true;
 }
@@ -652,6 +662,7 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
   constexpr bool UPW_ONLY = LES && (FLUX & FLUX_SIGMA0) != 0;
   constexpr bool IEEE = (FLUX & FLUX_IEEE) != 0;
   using D = DenOf<R, IEEE>;
+  using FD = FlushDenOf<R, IEEE>;
   R Fw[5], Ufw = R(0);
 #pragma unroll
   for (int q = 0; q < 5; q++) Fw[q] = R(0);
@@ -737,8 +748,8 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
         pL = eno_l(P[1], P[2], P[3], ord);
       } else {
   #pragma unroll
-        for (int q = 0; q < 5; q++) QL[q] = weno3_l<R, D>(Q[0][q], Q[1][q], Q[2][q]);
-        pL = weno3_l<R, D>(P[0], P[1], P[2]);
+        for (int q = 0; q < 5; q++) QL[q] = weno3_l<R, FD>(Q[0][q], Q[1][q], Q[2][q]);
+        pL = weno3_l<R, FD>(P[0], P[1], P[2]);
         if (!LES && !PLAIN && d == 1 && gj == 1 && c.isothermal && c.bctype[2] == 1) {  // rhs.c:2926
           QL[0] = eno_l(Q[1][0], Q[2][0], Q[3][0], ord);
           QL[4] = eno_l(Q[1][4], Q[2][4], Q[3][4], ord);
@@ -751,8 +762,8 @@ __device__ __forceinline__ void conv_face(const DevCfg &c, const DevFields &F, c
         pR = eno_r(P[0], P[1], P[2], ord);
       } else {
   #pragma unroll
-        for (int q = 0; q < 5; q++) QR[q] = weno3_r<R, D>(Q[1][q], Q[2][q], Q[3][q]);
-        pR = weno3_r<R, D>(P[1], P[2], P[3]);
+        for (int q = 0; q < 5; q++) QR[q] = weno3_r<R, FD>(Q[1][q], Q[2][q], Q[3][q]);
+        pR = weno3_r<R, FD>(P[1], P[2], P[3]);
       }
     }
     bool ok;

@@ -168,3 +168,84 @@ def test_sensor_beyond_the_quotients_range(kind):
         b.FormMetrics(coords)
         b.SetInitialCondition(q)
         assert _worst(b.formRHS(0), ref, far) <= RTOL_L2
+
+
+# ------------------------------------------------------------- mixed form ---
+# (ramp_e in the other schemes and heavy in the blend lie a little outside the form's bar whatever the quotients are)
+MIXED_CASES = ([("weno3_roe", "ramp_e")] + [(s, "heavy") for s in ("muscl", "muscl_roe")]
+               + [(s, "fine") for s in ("muscl_inviscid", "muscl_roe")])
+
+
+@pytest.mark.parametrize("scheme", ["weno3_blend", "weno5", "weno5_roe"])
+def test_mixed_weno_of_steep_energies_is_finite(scheme):
+    """The state ramp_e of the next test in the schemes that the bar leaves out."""
+    coords = W.periodic_grid(N, 2 * np.pi, amp=0.04)
+    shape = coords.shape[:3]
+    cfg = O.Config(mx=N[0] + 2, my=N[1] + 2, mz=N[2] + 2, ren=500.0, ma=0.3, pr=0.71, **{"inviscid": 0, **SCHEMES[scheme]})
+    q = W.random_smooth_state(shape, seed=9)
+    x = np.arange(shape[2])
+    q[..., 4] += 3.6e9 * np.minimum(x, shape[2] - 1 - x)
+    with gpu_block(cfg, precision="mixed") as b:
+        b.FormMetrics(coords)
+        b.SetInitialCondition(q)
+        if cfg.les and not cfg.inviscid:
+            b.CalcUCat()
+            b.Compute_eddy_viscosity_LES()
+        assert np.isfinite(b.formRHS(0)).all()
+
+
+@pytest.mark.parametrize("body", [False, True], ids=["clean", "body"])
+@pytest.mark.parametrize("scheme,kind", MIXED_CASES, ids=["-".join(c) for c in MIXED_CASES])
+def test_mixed_matches_the_restatement(scheme, kind, body):
+    """The mixed form's bar, 1e-5.  ramp_e: an energy that changes by 3.6e9 from node to node, so that every
+    (eps + beta)^2 lies in 2^126 .. 2^128, where the flushing reciprocal gives 0; heavy: densities of 1.0e38 .. 1.5e38,
+    above 2^126; fine: cells of 1.7e-10, whose squared face areas are subnormal."""
+    scale = 1.1e-9 if kind == "fine" else 1.0
+    coords = scale * W.periodic_grid(N, 2 * np.pi, amp=0.04)
+    shape = coords.shape[:3]
+    kw = {"inviscid": 0, **({"les": 0, "fluxorder": 2, "inviscid": 1} if scheme == "muscl_inviscid" else SCHEMES[scheme])}
+    cfg = O.Config(mx=N[0] + 2, my=N[1] + 2, mz=N[2] + 2, ren=500.0, ma=0.3, pr=0.71,
+                   dt={"ramp_e": 1e-8, "heavy": 1e-3, "fine": 1e-13}[kind], **kw)
+    q = W.random_smooth_state(shape, seed=9)
+    if kind == "ramp_e":
+        x = np.arange(shape[2])
+        q[..., 4] += 3.6e9 * np.minimum(x, shape[2] - 1 - x)
+    elif kind == "heavy":
+        rho, u = 1.5e38 * q[..., 0] / q[..., 0].max(), 0.3 * q[..., 1:4]
+        q[..., 0], q[..., 1:4] = rho, rho[..., None] * u
+        q[..., 4] = rho * (0.125 + 0.5 * (u * u).sum(axis=-1))
+    nv = np.zeros(shape)
+    if body:
+        nv[8:10, 7:9, 20:23] = 3.0
+    ref = oracle_run(cfg, coords, q, nv, steps=1)
+    assert np.isfinite(ref["rhs"]).all() and np.isfinite(ref["q_steps"]).all()
+    with gpu_block(cfg, precision="mixed") as b:
+        b.FormMetrics(coords)
+        if body:
+            b.set_nvert(nv)
+        b.SetInitialCondition(q)
+        if cfg.les and not cfg.inviscid:
+            b.CalcUCat()
+            b.Compute_eddy_viscosity_LES()
+        rhs = b.formRHS(0)
+        b.SetInitialCondition(q)
+        b.RungeKutta(1)
+        step = b.Q()
+    for got, want in ((rhs, ref["rhs"]), (step, ref["q_steps"])):
+        for f in range(5):
+            top = np.abs(want[..., f]).max()
+            assert O.rel_l2(got[..., f] / top, want[..., f] / top) <= 1e-5
+
+
+def test_mixed_eddy_viscosity_of_heavy_states():
+    coords = W.periodic_grid(N, 2 * np.pi, amp=0.04)
+    shape = coords.shape[:3]
+    cfg = O.Config(mx=N[0] + 2, my=N[1] + 2, mz=N[2] + 2, ren=500.0, ma=0.3, pr=0.71, inviscid=0, les=1)
+    q = _momentum(shape, 1.5e38, 0.3)
+    ref = oracle_run(cfg, coords, q, np.zeros(shape))["nut"]
+    with gpu_block(cfg, precision="mixed") as b:
+        b.FormMetrics(coords)
+        b.SetInitialCondition(q)
+        b.CalcUCat()
+        b.Compute_eddy_viscosity_LES()
+        assert O.rel_l2(b.nu_t(), ref) <= 1e-5
