@@ -11,12 +11,12 @@
 //   y0 ~ 1/b (rcp.approx, |1 - b y0| <= 2^-19.9 measured), e = 1 - b y0,
 //   y = y0 + y0 (e + e^2)                    -- the cubic step, error 2^-53
 //   q0 = a y,  r = a - b q0 (exact),  q = q0 + r y
-// q is the IEEE quotient unless a / b lies within 2^-51 ulp of a rounding
-// boundary (none of 1.05e9 random pairs differed from __ddiv_rn), in 3 FP64
+// q is the IEEE quotient unless a / b lies within 2^-52 ulp of a rounding
+// boundary (tests/test_gpu_quotients.py: random pairs, and pairs built from a
+// boundary; a power of two over a mantissa of ones is such a pair), in 3 FP64
 // operations per quotient after 3 for the reciprocal, with no branch, so the
 // chains of a face's quotients overlap.  The square root is the same
-// correction of a Goldschmidt iterate (none of 1.05e9 differed from
-// __dsqrt_rn).  Measured per time step, before and after, with bit-identical
+// correction of a Goldschmidt iterate (IEEE unless within 2^-50 ulp of one).  Measured per time step, before and after, with bit-identical
 // results: MUSCL + Rusanov 128^3 1.50 -> 1.36 ms, WENO3 blend 97x75x61
 // 1.60 -> 1.00 ms, WENO5-JS + Roe 96^3 4.22 -> 2.86 ms, inviscid WENO5-JS +
 // Rusanov 64^3 1.08 -> 0.63 ms; mixed form (the node reciprocal only) WENO5-JS
