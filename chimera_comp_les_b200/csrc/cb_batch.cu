@@ -358,6 +358,9 @@ int cb_batch_create(const cb_config *cfg, int nblocks, const int *dims, cb_batch
   if (cfg->weno_order == 5 && cfg->fluxorder != 3) return bail(CB_E_ARG, "weno_order 5 needs fluxorder 3");
   if (cfg->visT && !(cfg->tref > 0.0)) return bail(CB_E_ARG, "Tref must be > 0 with visT");
   if (batch_dynamic(*cfg) && !(cfg->max_cs >= 0.0)) return bail(CB_E_ARG, "max_cs must be >= 0");
+  for (int k = 0; k < nblocks; k++)  // (a product of doubles: no overflow for any three ints)
+    if ((dims[3 * k] + 4.0) * (dims[3 * k + 1] + 4.0) * (dims[3 * k + 2] + 4.0) >= 2147483648.0)
+      return bail(CB_E_ARG, "block too large for 32-bit node indexing");
   b->dev = cfg->device;
   if (cudaSetDevice(b->dev) != cudaSuccess) return bail(CB_E_CUDA, "cudaSetDevice");
   cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->dev);
@@ -395,7 +398,6 @@ int cb_batch_create(const cb_config *cfg, int nblocks, const int *dims, cb_batch
     d.abc = cfg->abc;
     d.flux = cfg->flux;
     d.twall = cfg->twall;
-    if (shell_count(d) >= (1LL << 31)) return bail(CB_E_ARG, "block too large for 32-bit boundary indexing");
     bh.off = off;
     off += (d.plane + 31) / 32 * 32;  // 256-byte aligned block starts
     bh.tiles_x = (bh.mx - 2 + SBX - 1) / SBX;
