@@ -1741,7 +1741,7 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
 // planes beside dirty ones stays with them: a piece of its own costs a
 // prologue, about one plane.
 constexpr int MASK_MIN_RUN = 5;
-template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX, bool NV0>
+template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX, bool NV0, bool CLEAN>
 __device__ __forceinline__ void stage_block(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta,
                                             double adt, int kchunk, double *smem_d, int *again) {
   constexpr int BY = StageGeo<FLUX>::BY;
@@ -1762,7 +1762,7 @@ __device__ __forceinline__ void stage_block(const DevCfg &c, const DevFields &F,
     const int col = (int)(s / nk), k0 = (int)(s - (long long)col * nk);
     int k1 = (int)min((long long)nk, k0 + (e - s));
     bool clean = NV0;
-    if constexpr (!NV0 && (FLUX & FLUX_IEEE) == 0) {
+    if constexpr (!NV0 && CLEAN) {
       int lo = 0, hi = nk;  // dirty planes lo .. hi - 1 of the column
       if (F.mask_planes != nullptr) { const int2 d = F.mask_planes[col]; lo = d.x; hi = d.y; }
       else if (F.all_clean) hi = 0;
@@ -1772,7 +1772,7 @@ __device__ __forceinline__ void stage_block(const DevCfg &c, const DevFields &F,
       else if (lo - k0 >= MASK_MIN_RUN) { clean = true; k1 = lo; }
       else if (k1 - hi >= MASK_MIN_RUN) k1 = hi;
     }
-    if constexpr (NV0 || (FLUX & FLUX_IEEE) == 0)
+    if constexpr (NV0 || CLEAN)
       if (clean)
         stage_tile<R, MIX, LES, VISC, RHS_MODE, FLUX, true>(c, F, col % tiles_x, col / tiles_x, 1 + k0, 1 + k1, istage,
                                                             alfa, beta, adt, smem_d, again);
@@ -1791,7 +1791,7 @@ template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX, bo
 static __device__ __noinline__ void stage_again(const DevCfg &c, const DevFields &F, int istage, double alfa, double beta,
                                                 double adt, int kchunk) {
   extern __shared__ double smem_d[];
-  stage_block<R, MIX, LES, VISC, RHS_MODE, FLUX, NV0>(c, F, istage, alfa, beta, adt, kchunk, smem_d, nullptr);
+  stage_block<R, MIX, LES, VISC, RHS_MODE, FLUX, NV0, false>(c, F, istage, alfa, beta, adt, kchunk, smem_d, nullptr);
 }
 __host__ __device__ constexpr int ieee_flux(int fl, bool blend) { return FLUX_IEEE | (blend ? FLUX_BLEND : 0) | (fl & (FLUX_ROE | FLUX_W5)); }
 
@@ -1801,7 +1801,9 @@ __host__ __device__ constexpr int ieee_flux(int fl, bool blend) { return FLUX_IE
 // results are overwritten.  The call stands at the kernel's end, where no value
 // lives across it (inside the loop over the tiles: MUSCL 128^3 3 % slower,
 // WENO5-JS + Roe 96^3 10 %).
-template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX = 0, bool NV0 = false>
+// CLEAN: the split of columns into planes with and without nvert (a caller that
+// never has the lists, cb_rhs_noalloc, goes without that code).
+template <typename R, bool MIX, bool LES, bool VISC, bool RHS_MODE, int FLUX = 0, bool NV0 = false, bool CLEAN = true>
 static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThreads<FLUX, MIX>::MIN_BLOCKS)
     stage_kernel(const __grid_constant__ DevCfg c, const __grid_constant__ DevFields F, int istage, double alfa, double beta,
                  double adt, int kchunk) {
@@ -1812,7 +1814,7 @@ static __global__ void __launch_bounds__(StageThreads<FLUX, MIX>::N, StageThread
     __syncthreads();
   }
   pdl_wait();
-  stage_block<R, MIX, LES, VISC, RHS_MODE, FLUX, NV0>(c, F, istage, alfa, beta, adt, kchunk, smem_d, &again);
+  stage_block<R, MIX, LES, VISC, RHS_MODE, FLUX, NV0, CLEAN>(c, F, istage, alfa, beta, adt, kchunk, smem_d, &again);
   if constexpr (!MIX)
     if (again)  // (every march ends with a barrier)
       stage_again<R, MIX, LES, VISC, RHS_MODE, ieee_flux(FLUX, RHS_MODE), NV0>(c, F, istage, alfa, beta, adt, kchunk);
@@ -1903,12 +1905,12 @@ inline int stage_threads(int fl) {
   return (fl & FLUX_W5) ? StageThreads<FLUX_W5, MIX>::N : StageThreads<0, MIX>::N;
 }
 template <typename R, bool MIX>
-size_t stage_smem_for(int fl, bool nv0) {
+size_t stage_smem_for(int fl, bool nv0, bool both = true) {
   const bool w5 = (fl & FLUX_W5) != 0;
   const size_t clean = w5 ? stage_smem<R, MIX, true, true>() : stage_smem<R, MIX, true, false>();
   const size_t gen = w5 ? stage_smem<R, MIX, false, true>() : stage_smem<R, MIX, false, false>();
-  // a kernel with nvert runs both kinds of tile (the batched one only its own)
-  return nv0 ? clean : (clean > gen ? clean : gen);
+  // a kernel with nvert runs both kinds of tile, the batched one only its own
+  return nv0 ? clean : (both && clean > gen ? clean : gen);
 }
 // Opt every variant of one (LES, VISC, RHSM) into its dynamic shared memory.
 template <typename R, bool MIX, bool LES, bool VISC, bool RHSM>

@@ -104,7 +104,7 @@ cudaError_t batched_attrs() {
   cudaError_t e = cudaSuccess;
   for (int fl : {0, FLUX_ROE, FLUX_W5, FLUX_ROE | FLUX_W5})
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(batched_kernel<R, MIX, LES, VISC>(fl, false), attr, (int)stage_smem_for<R, MIX>(fl, false));
+      e = cudaFuncSetAttribute(batched_kernel<R, MIX, LES, VISC>(fl, false), attr, (int)stage_smem_for<R, MIX>(fl, false, false));
   for (int w : {0, FLUX_W5, FLUX_PLAIN, FLUX_PLAIN | FLUX_W3, FLUX_W5 | FLUX_PLAIN})
     for (int fl = 0; fl < (LES ? 6 : 2) && e == cudaSuccess; fl++)
       e = cudaFuncSetAttribute(batched_kernel<R, MIX, LES, VISC>(w | fl, true), attr,
@@ -122,7 +122,7 @@ template <typename R, bool MIX, bool LES, bool VISC>
 cudaError_t BatchLaunch<R, MIX, LES, VISC>::launch(const BatchBlock *tab, const int2 *items, int nitems, unsigned *counter,
                                                    int istage, double alfa, double beta, double adt, int fl, bool nv0,
                                                    int ctas, cudaStream_t s) {
-  batched_kernel<R, MIX, LES, VISC>(fl, nv0)<<<ctas, stage_threads<MIX>(fl), stage_smem_for<R, MIX>(fl, nv0), s>>>(
+  batched_kernel<R, MIX, LES, VISC>(fl, nv0)<<<ctas, stage_threads<MIX>(fl), stage_smem_for<R, MIX>(fl, nv0, false), s>>>(
       tab, items, nitems, counter, istage, alfa, beta, adt);
   return cudaGetLastError();
 }
