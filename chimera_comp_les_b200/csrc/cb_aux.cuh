@@ -749,8 +749,10 @@ static inline dim3 eddy_grid(const DevCfg &c, int kchunk) {
 
 // ------------------------------------------------------------ shock sensor --
 // Hybrid weights with -calc_sigma (formConvectionLES at istage 0,
-// rhs.c:3328-3433; compute_ri / sigma_cent rhs.c:2334-2358).  Three passes
-// with a ghost fill between them, as the reference's DMGlobalToLocal calls:
+// rhs.c:3328-3433; compute_ri / sigma_cent rhs.c:2334-2358).  Three passes;
+// the reference wraps the weights after each, but no pass reads one beyond the
+// owned nodes, and a single block forms no such ghosts (a batch fills them by
+// its donor maps):
 // raw ramp per direction, product filter of neighbour square roots,
 // curvature rule with y = z = min(y, z).  Boundary nodes keep (s_x, s_y, s_z).
 __device__ __forceinline__ double sensor_ri(double fR, double f0, double fL, double ks) {
@@ -811,7 +813,7 @@ static __global__ void sigma_sensor_kernel(const DevCfg c, const double *const *
   }
 }
 
-// pass 2 (ls: ghosted pass-1 planes): interior nodes times
+// pass 2 (ls: pass-1 planes): interior nodes times
 // sqrt(ls[j-1] ls) sqrt(ls[k-1] ls[k+1]) sqrt(ls[i-1] ls[i+1]); others copied
 static __global__ void sigma_filter_kernel(const DevCfg c, const double *const *ls, double *const *sig) {
   pdl_wait();
@@ -832,7 +834,7 @@ static __global__ void sigma_filter_kernel(const DevCfg c, const double *const *
   }
 }
 
-// pass 3 (ls: ghosted pass-2 planes): curvature rule, then y = z = min(z, y)
+// pass 3 (ls: pass-2 planes): curvature rule, then y = z = min(z, y)
 static __global__ void sigma_post_kernel(const DevCfg c, const double *const *ls, double *const *sig) {
   pdl_wait();
   const long long total = (long long)c.px * c.py * c.pz;

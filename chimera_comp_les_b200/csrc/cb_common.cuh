@@ -122,7 +122,8 @@ __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefe
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // (i, j, k) of element t of an nx x ny x nz box, i fastest: 32-bit division
-// (the hosts check that every box stays below 2^32 elements), which takes a
+// (cb_create and cb_batch_create keep (mx+4)(my+4)(mz+4) below 2^31, so the box
+// with its padded rows stays below 2^32; cb_rhs_noalloc's is smaller), which takes a
 // fifth of the instructions of the 64-bit one
 __device__ __forceinline__ void split3(unsigned t, int nx, int ny, int &i, int &j, int &k) {
   const unsigned r = t / (unsigned)nx, s = r / (unsigned)ny;

@@ -15,12 +15,12 @@
 // boundary (tests/test_gpu_quotients.py: random pairs, and pairs built from a
 // boundary; a power of two over a mantissa of ones is such a pair), in 3 FP64
 // operations per quotient after 3 for the reciprocal, with no branch, so the
-// chains of a face's quotients overlap.  The square root is the same
-// correction of a Goldschmidt iterate (IEEE unless within 2^-50 ulp of one).  Measured per time step, before and after, with bit-identical
-// results: MUSCL + Rusanov 128^3 1.50 -> 1.36 ms, WENO3 blend 97x75x61
-// 1.60 -> 1.00 ms, WENO5-JS + Roe 96^3 4.22 -> 2.86 ms, inviscid WENO5-JS +
-// Rusanov 64^3 1.08 -> 0.63 ms; mixed form (the node reciprocal only) WENO5-JS
-// + Roe 192^3 7.97 -> 7.85 ms.
+// chains of a face's quotients overlap.  The square root is the same correction
+// of a Goldschmidt iterate (IEEE unless within 2^-50 ulp of one).  Measured per
+// time step, before and after, with bit-identical results: MUSCL + Rusanov 128^3
+// 1.50 -> 1.36 ms, WENO3 blend 97x75x61 1.60 -> 1.00 ms, WENO5-JS + Roe 96^3
+// 4.22 -> 2.86 ms, inviscid WENO5-JS + Rusanov 64^3 1.08 -> 0.63 ms; mixed form
+// (the node reciprocal only) WENO5-JS + Roe 192^3 7.97 -> 7.85 ms.
 //
 // Range: that holds for denominators and radicands with |b| in 2^-960 .. 2^960
 // (in_range) and finite numerators whose quotient does not overflow; below

@@ -1156,10 +1156,9 @@ __device__ __forceinline__ void face_flux_half(const DevCfg &c, const DevFields 
 
 // ---------------------------------------------------------- the kernel ----
 // Tile of 32 x BY interior nodes, NT = 32 (BY + 1) threads (StageGeo).  Per
-// plane the block computes 33*BY i-faces, 32*(BY+1) j-faces and 32*BY k-faces
-// in three warp-uniform rounds: virtual face v = round*NT + tid maps to
-// [0,NT) i-faces, [NT,2NT) j-faces, [2NT,3NT) k-faces, so every warp runs one
-// face direction per round (no divergence between directions).
+// plane the block computes 33*BY i-faces, 32*(BY+1) j-faces and 32*BY k-faces:
+// the mixed form in three rounds of NT threads, a direction each, the FP64 form
+// in the jobs of plane_faces; every warp runs one face direction at a time.
 constexpr int SBX = 32, SBY = StageGeo<0>::BY, SNT = StageGeo<0>::NT;  // the WENO3/MUSCL tile: 32 x 7, 256 threads
 constexpr int SBY_W5 = StageGeo<FLUX_W5>::BY, SNT_W5 = StageGeo<FLUX_W5>::NT;  // WENO5: 32 x 5, 192 threads
 template <typename R, bool MIX, bool NV0 = false, bool W5 = false>
@@ -1388,10 +1387,9 @@ __device__ __forceinline__ void stage_tile(const DevCfg &c, const DevFields &F, 
   // buffer: node-major, one index computation per node and one 8-byte copy
   // per staged field (consecutive threads take consecutive nodes of a row, so
   // each field's copies stay coalesced)
-  // In the FP64 form the threads of the inviscid half issue the copies and
-  // those of the viscous half run the derive pass: the viscous face takes
-  // longer, and the inviscid threads also run the node update, in the same
-  // phase as the derive pass.
+  // In the FP64 form the first half of the block issues the copies and runs the
+  // node update, and the second half the derive pass, in the same phase as the
+  // update.
   constexpr bool SPLIT = StageThreads<FLUX, MIX>::SPLIT;
   constexpr int HT = SPLIT ? NT / 2 : NT;  // threads of one half
   auto issue_stage = [&](int kk) {
