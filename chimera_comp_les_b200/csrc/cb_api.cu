@@ -540,7 +540,7 @@ int cb_create(const cb_config *cfg, cb_ctx **out) {
   if (cudaSetDevice(c->dev) != cudaSuccess) return bail(CB_E_CUDA, "cudaSetDevice failed");
   cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(CB_E_CUDA, "stream");
-  if (stage_attrs_all(cfg->precision == CB_MIXED) != cudaSuccess)
+  if (stage_attrs_for(cfg->precision == CB_MIXED, cfg->les != 0, cfg->inviscid == 0) != cudaSuccess)
     return bail(CB_E_CUDA, "stage kernel shared-memory opt-in failed");
   DevCfg &d = c->dc;
   d.mx = cfg->mx; d.my = cfg->my; d.mz = cfg->mz;

@@ -469,7 +469,8 @@ int cb_batch_create(const cb_config *cfg, int nblocks, const int *dims, cb_batch
   }
   {
     const bool mix = cfg->precision == CB_MIXED;
-    if (stage_attrs_all(mix) != cudaSuccess || batch_attrs_all(mix) != cudaSuccess)
+    if (stage_attrs_for(mix, cfg->les != 0, cfg->inviscid == 0) != cudaSuccess ||
+        batch_attrs_for(mix, cfg->les != 0, cfg->inviscid == 0) != cudaSuccess)
       return bail(CB_E_CUDA, "stage kernel attributes");
   }
   if (cudaMalloc(&b->staging, sizeof(double) * 5 * maxnn) != cudaSuccess) return bail(CB_E_CUDA, "staging");

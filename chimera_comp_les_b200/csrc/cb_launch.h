@@ -71,16 +71,14 @@ inline cudaError_t with_part(bool mix, bool les, bool visc, Fn f) {
   if (les) return visc ? f(L<double, false, true, true>{}) : f(L<double, false, true, false>{});
   return visc ? f(L<double, false, false, true>{}) : f(L<double, false, false, false>{});
 }
-template <template <typename, bool, bool, bool> class L>
-inline cudaError_t attrs_all(bool mix) {
-  cudaError_t e = cudaSuccess;
-  for (bool les : {true, false})
-    for (bool visc : {true, false})
-      if (e == cudaSuccess) e = with_part<L>(mix, les, visc, [](auto p) { return decltype(p)::attrs(); });
-  return e;
+// the shared-memory opt-in of a context's part alone, since it loads the part's
+// kernels (a process's first FP64 context: 75-170 ms, with all four parts 185-440)
+inline cudaError_t stage_attrs_for(bool mix, bool les, bool visc) {
+  return with_part<StageLaunch>(mix, les, visc, [](auto p) { return decltype(p)::attrs(); });
 }
-inline cudaError_t stage_attrs_all(bool mix) { return attrs_all<StageLaunch>(mix); }
-inline cudaError_t batch_attrs_all(bool mix) { return attrs_all<BatchLaunch>(mix); }
+inline cudaError_t batch_attrs_for(bool mix, bool les, bool visc) {
+  return with_part<BatchLaunch>(mix, les, visc, [](auto p) { return decltype(p)::attrs(); });
+}
 inline cudaError_t launch_stage_any(bool mix, bool les, const DevCfg &c, const DevFields &F, int istage, double alfa,
                                     double beta, double adt, int kchunk, bool visc, bool rhs_mode, int fl, bool nv0,
                                     int slots, cudaStream_t s) {
